@@ -150,8 +150,9 @@ typedef struct mgfvm_tuning {
                                               sweeps) per tile launch, >= 1             */
     int smooth_threads[MGFVM_MAX_LEVELS];  /* smoother CTA: 1024 (one per SM), 512 (two)
                                               or 256 threads (four)                     */
-    int asm_slices[MGFVM_MAX_LEVELS];      /* assembly threads per cell: 1 or 3         */
-    int restrict_slices[MGFVM_MAX_LEVELS]; /* restriction threads per cell: 1 or 3      */
+    int asm_slices[MGFVM_MAX_LEVELS];      /* assembly threads per cell, 1 or 3, that share
+                                              nothing; 0: by tiles through shared memory */
+    int restrict_slices[MGFVM_MAX_LEVELS]; /* the same for the restriction              */
     int update_pfix[MGFVM_MAX_LEVELS];     /* obstacle pressure copy inside update where
                                               legal: 0 or 2 yes, 1 no (own kernel)      */
     int odd_chunks[MGFVM_MAX_LEVELS];      /* an odd number of tile-smoother launches may

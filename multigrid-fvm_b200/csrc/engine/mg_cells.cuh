@@ -289,7 +289,7 @@ __device__ __forceinline__ typename IO::T mass_coefp_io(const IO &io, const Case
                                                         int vs, int parts = MC_ALL)
 {
     using T = typename IO::T;
-    const LevelDev &L = io.L;
+    const auto &L = io.L;
     const int nx = L.npx, ny = L.npy, q = j * nx + i, s = q - nx;
     const double axq = io.g(S_AREAX, q), ayq = io.g(S_AREAY, q);
     T div = T(0.0), su = T(0.0);
@@ -403,33 +403,60 @@ __device__ __forceinline__ T gs_value(const T &aw, const T &ae, const T &as, con
 // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., sec. 4.7):
 // q0 = RN(a y); r0 = a - b q0 and q1 = RN(q0 + r0 y) make q1 faithful (|q1 - a/b| <
 // ulp), so r1 = a - b q1 is exact and q2 = RN(q1 + r1 y) = RN(a/b).  The theorem needs
-// no underflow or overflow anywhere: operands outside [2^-450, 2^450] in magnitude
-// (which keeps the quotient within [2^-900, 2^900]), zero, Inf and NaN take the IEEE
-// division.  Results are therefore the bits of a / b in every case.
+// no underflow or overflow anywhere: operands outside [2^-450, 2^450) in magnitude
+// (which keeps the quotient within [2^-900, 2^900]), zero divisors, Inf and NaN take the
+// IEEE division, except the two dividends that fill the inside of obstacles, where the
+// 1e30 diagonals drive values down by 1e-30 a cell: a zero's quotient is q0, whose sign is
+// the division's, and a tiny one is divided after scaling by 2^600 (exact) and scaled back,
+// exact where the quotient is normal and a correctly signed zero where it is below half the
+// smallest subnormal; only subnormal quotients are left to the IEEE division.  Results are
+// therefore the bits of a / b in every case.  (The compiled IEEE division takes a slow path
+// for such dividends.)  The ranges are tested on the high words, off the FP64 pipe; a recip with y = 0 stands for
+// a divisor out of range.
 struct Recip {
     double b, y;
-    bool ok;
 };
+
+// |x| in [2^lo, 2^hi)
+template <int LO, int HI>
+__device__ __forceinline__ bool exponent_in(double x)
+{
+    return (unsigned)((__double2hiint(x) & 0x7fffffff) - ((1023 + LO) << 20)) < (unsigned)((HI - LO) << 20);
+}
 
 __device__ __forceinline__ Recip make_recip(double b)
 {
-    const double m = fabs(b);
-    return {b, 1.0 / b, m >= 0x1p-450 && m <= 0x1p450};
+    const double y = 1.0 / b;
+    return {b, exponent_in<-450, 450>(b) ? y : 0.0};
 }
 
-__device__ __forceinline__ double ieee_div(double a, double b) { return a / b; }
+__device__ __forceinline__ double markstein(double a, const Recip &R)
+{
+    const double q0 = a * R.y;
+    const double r0 = fma(-R.b, q0, a);
+    const double q1 = fma(r0, R.y, q0);
+    const double r1 = fma(-R.b, q1, a);
+    return fma(r1, R.y, q1);
+}
+
+// div_by's operands outside the plain range (a call: inlined at every division it would
+// crowd the instruction cache)
+static __device__ __noinline__ double div_by_rare(double a, double b, double y)
+{
+    if (__double2hiint(y) != 0) {
+        if (a == 0.0) return a * y;
+        if (fabs(a) < 0x1p-450) {
+            const double q = markstein(a * 0x1p600, Recip{b, y});
+            if (exponent_in<-422, 1023>(q) || fabs(q) < 0x1p-476) return q * 0x1p-600;
+        }
+    }
+    return a / b;
+}
 
 __device__ __forceinline__ double div_by(double a, const Recip &R)
 {
-    const double m = fabs(a);
-    if (R.ok && m >= 0x1p-450 && m <= 0x1p450) {
-        const double q0 = a * R.y;
-        const double r0 = fma(-R.b, q0, a);
-        const double q1 = fma(r0, R.y, q0);
-        const double r1 = fma(-R.b, q1, a);
-        return fma(r1, R.y, q1);
-    }
-    return ieee_div(a, R.b);
+    if (exponent_in<-450, 450>(a) && __double2hiint(R.y) != 0) return markstein(a, R);
+    return div_by_rare(a, R.b, R.y);
 }
 
 // gs_value with the divisor's reciprocal precomputed (R = make_recip(ap))

@@ -46,7 +46,9 @@ struct LevelDev {
     int npx, npy;
     int ncopy;          // pressure-copy program length (update's obstacle loop)
     int hazard;         // the copy program reads a cell it also writes
+    unsigned sb;        // f[s] = f[0] + s * sb bytes (the slots of a level lie at one stride)
     double dx, dy;
+    double rdx, rdy;    // their reciprocals for div_by (0 where dx, dy are outside its range)
     double amu;         // viscosity on this level (amuf, :419)
     double amusc;       // scalar diffusivity amuf/prsc (:867)
     double *f[NSLOTS];
@@ -74,6 +76,7 @@ enum CaseStatus { CASE_RUNNING = 0, CASE_CONVERGED_REF = 1, CASE_CONVERGED_FP = 
 struct CaseDev {
     // physics and boundary codes shared by every level (Version-6-26-04.c:30-35)
     double relxm, relxp, sc_obs, dpdxm, dpdym, convergence;
+    double rrelxm;      // reciprocal of relxm for div_by
     int ibc_xm, ibc_xp, ibc_ym, ibc_yp;
     int ngrid;
     int tail;           // first level run by the one-CTA coarse kernel (== ngrid: none)

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mg_adjoint.cuh"
+#include "mg_fast.cuh"
 #include "mg_init.cuh"
 #include "mg_kernels.cuh"
 #include "mg_tangent.cuh"
@@ -104,6 +105,13 @@ static inline int npx_of(const mgfvm_config &c, int ig) { return c.nfx / (1 << i
 static inline int npy_of(const mgfvm_config &c, int ig) { return c.nfy / (1 << ig) + 2; }
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 static inline int nblk(long long n) { return (int)std::max<long long>(1, (n + BLOCK - 1) / BLOCK); }
+
+// the reciprocal y of a Recip (mg_cells.cuh) with divisor b, 0 outside its range
+static double recip_of(double b)
+{
+    const double m = std::fabs(b);
+    return m >= 0x1p-450 && m < 0x1p450 ? 1.0 / b : 0.0;
+}
 
 // ------------------------------------------------------------------ schedule
 namespace {
@@ -204,6 +212,14 @@ struct Builder {
                 m = std::max(m, ((w + tile - 1) / tile) * ((h + tile - 1) / tile));
             }
         return std::max<long long>(m, 1);
+    }
+    // Tiles of the level's padded grid, less `ring` cells in each direction, at most over the cases.
+    int grid_tiles(int ig, int ring) const
+    {
+        int m = 1;
+        for (const mgfvm_config &c : x->cfg)
+            if (ig < c.ngrid) m = std::max(m, tiles_of(npx_of(c, ig) - ring, npy_of(c, ig) - ring));
+        return m;
     }
     // Whether one CTA per (case, equation) holds the level: its padded grid has at
     // most SMOOTH_BLOCK vertical cell pairs in every case.
@@ -469,9 +485,8 @@ struct Builder {
     // on the visit-start fluxes, so they are assembled together and smoothed in the
     // same launches; the scalar's outflow ghost moves with its equation.
     static int asm_bits(bool down) { return A_FLUX | A_U | A_V | A_SC | (down ? A_SC_OUTFLOW : 0); }
-    // Assembly and restriction run one thread per (cell, equation) — 3 slices, each
-    // with a third of the dependent loads — unless tuned to one thread per cell.
-    static int slices(int, int knob) { return knob == 1 ? 1 : 3; }
+    // Assembly and restriction run by tiles, one thread a cell, unless tuned to 1 or 3 thread
+    // slices a cell that share nothing.
     // the assembly bits of a down-leg (or up-leg) step on level ig, with the FP32
     // operands of a mixed-precision level
     int asm_what(int ig, int mode, bool down) const
@@ -519,8 +534,10 @@ struct Builder {
             return;
         }
         if (!asm_done) {
-            Launch &L = add(K_ASM, ig, mode, cells(ig), asm_what(ig, mode, down), 1);
-            L.grid.z = slices(ig, x->tune.asm_slices[ig]);
+            const int z = x->tune.asm_slices[ig];
+            Launch &L = add(K_ASM, ig, mode, cells(ig), asm_what(ig, mode, down), z ? 1 : 2);
+            if (z) L.grid.z = z;
+            else L.grid.x = grid_tiles(ig, 0);
         }
         const bool in_tmp = smooth(ig, mode, (1 << EQ_U) | (1 << EQ_V) | (1 << EQ_SC), x->sched.nswpm,
                                    x->tune.odd_chunks[ig] != 1);
@@ -532,10 +549,13 @@ struct Builder {
     // `coarse_asm`: also run the coarse level's down-leg assembly (see k_restrict)
     void restrict_(int ig, int mode_f, bool coarse_asm = false)
     {
-        const int z = slices(ig, x->tune.restrict_slices[ig]);
-        add(K_RESTV_FLUXES, ig, mode_f, cells(ig)).grid.z = z;
-        Launch &L = add(K_RESTRICT, ig, mode_f, cells(ig + 1), coarse_asm ? asm_what(ig + 1, M_DOWN, true) : 0);
-        L.grid.z = z;
+        const int z = x->tune.restrict_slices[ig], what = coarse_asm ? asm_what(ig + 1, M_DOWN, true) : 0;
+        Launch &R = add(K_RESTV_FLUXES, ig, mode_f, cells(ig), 0, z ? 0 : 2);
+        if (z) R.grid.z = z;
+        else R.grid.x = grid_tiles(ig, 2);
+        Launch &L = add(K_RESTRICT, ig, mode_f, cells(ig + 1), what, z ? 0 : 2);
+        if (z) L.grid.z = z;
+        else L.grid.x = grid_tiles(ig + 1, 0);
     }
     // :230-233
     // In a V-cycle the gather may form the coarse corrections from the R(x_f) that the
@@ -544,7 +564,7 @@ struct Builder {
     {
         const bool fused = mode == M_PROLONG && x->tune.prol_fused[ig] != 1;
         if (!fused) add(K_PROL_CORR, ig, mode, cells(ig + 1));
-        add(K_PROL_APPLY, ig, mode, cells(ig), fused ? 1 : 0);
+        add(K_PROL_APPLY, ig, mode, cells(ig), fused ? 1 : 0).grid.x = grid_tiles(ig, 2);
     }
     // The first level of the coarse cluster launch (k_coarse_cycle, when the tuning asks
     // for it): the first level one CTA per case holds, when every level from there down
@@ -1188,7 +1208,7 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
             pend.push_back(p);
         }
         const long long n0 = (long long)(npx_of(g, 0) - 2) * (npy_of(g, 0) - 2);
-        part_off[c] = take((size_t)std::max(nblk(n0), 64) * RED_STRIDE * sizeof(double));
+        part_off[c] = take((size_t)std::max({nblk(n0), tiles_of(npx_of(g, 0) - 2, npy_of(g, 0) - 2), 64}) * RED_STRIDE * sizeof(double));
         cnt_off[c] = take(16 * sizeof(unsigned));
     }
     const size_t pool_bytes = align_up(off, 256);
@@ -1204,6 +1224,7 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         const mgfvm_config &g = x->cfg[c];
         C.relxm = g.relxm; C.relxp = g.relxp; C.sc_obs = g.sc_obs;
         C.dpdxm = g.dpdxm; C.dpdym = g.dpdym; C.convergence = g.convergence;
+        C.rrelxm = recip_of(g.relxm);
         C.ibc_xm = g.ibc_xm; C.ibc_xp = g.ibc_xp; C.ibc_ym = g.ibc_ym; C.ibc_yp = g.ibc_yp;
         C.ngrid = g.ngrid;
         int tail = g.ngrid;
@@ -1225,9 +1246,17 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         L.npy = npy_of(g, p.ig);
         L.dx = g.xl / (L.npx - 2);       // AllocateMemorySoA :413-414
         L.dy = g.yl / (L.npy - 2);
+        L.rdx = recip_of(L.dx);
+        L.rdy = recip_of(L.dy);
         L.amu = g.amuf;
         L.amusc = g.amuf / g.prsc;       // coefsc :867
         for (int s = 0; s < NSLOTS; ++s) L.f[s] = p.slot[s] == (size_t)-1 ? nullptr : (double *)(x->pool + p.slot[s]);
+        const size_t sb = p.slot[1] - p.slot[0];
+        for (int s = 0; s < NSLOTS; ++s)
+            if (p.slot[s] != (size_t)-1 && p.slot[s] != p.slot[0] + s * sb)
+                return mgfvm_fail(MGFVM_EUNSUPPORTED, "level arrays not at one stride");
+        if (sb > 0xffffffffull) return mgfvm_fail(MGFVM_ENOMEM, "a level array of %zu bytes", sb);
+        L.sb = (unsigned)sb;
         L.tag = (int *)(x->pool + p.tag);
         const mgfvm_obstacle_prog &P = x->progs[(size_t)p.c * MAXLEV + p.ig];
         L.ncopy = P.ncopy;

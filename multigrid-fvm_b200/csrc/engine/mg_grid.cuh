@@ -1,0 +1,72 @@
+// mg_grid.cuh — index domains, programmatic launch and launch helpers shared by the
+// engine's kernel files.
+#pragma once
+
+#include "mg_cells.cuh"
+
+namespace mg {
+
+struct Dom { int i0, j0, wi, wj; };
+
+static __device__ __forceinline__ Dom dom_all(const LevelDev &L) { return {0, 0, L.npx, L.npy}; }
+static __device__ __forceinline__ Dom dom_interior(const LevelDev &L) { return {1, 1, L.npx - 2, L.npy - 2}; }
+static __device__ __forceinline__ Dom dom_flux(const LevelDev &L) { return {0, 0, L.npx - 1, L.npy - 1}; }
+// sweep extent of each equation (solve_u/v/pprime/sc :701, :710, :725, :735)
+static __device__ __forceinline__ Dom dom_eq(const LevelDev &L, int e)
+{
+    if (e == EQ_U) return {1, 1, L.npx - 3, L.npy - 2};
+    if (e == EQ_V) return {1, 1, L.npx - 2, L.npy - 3};
+    return dom_interior(L);
+}
+
+static __device__ __forceinline__ bool cell_at(const Dom &d, int t, int &i, int &j)
+{
+    if (d.wi <= 0 || d.wj <= 0 || t >= d.wi * d.wj) return false;
+    j = d.j0 + t / d.wi;
+    i = d.i0 + t % d.wi;
+    return true;
+}
+
+static __device__ __forceinline__ int nth_eq(int mask, int k)
+{
+    for (int e = 0; e < 4; ++e)
+        if ((mask >> e) & 1) {
+            if (k == 0) return e;
+            --k;
+        }
+    return -1;
+}
+
+// ---------------------------------------------- programmatic dependent launch
+// The V-cycle's kernels are launched with programmatic stream serialization (when the
+// schedule's `pdl` switch is on), so a kernel's CTAs may be scheduled while its
+// predecessor is still running.  Every kernel therefore starts by waiting until the
+// grids it depends on have completed and their memory is visible (a no-op for a
+// kernel launched without the attribute), and then lets its own dependent launch
+// begin: at most one kernel waits ahead of the running one, and nothing a kernel
+// reads or writes is touched before its predecessors are done.
+static __device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch `k` on `st`, with programmatic stream serialization when `pdl` (the kernel
+// may then be scheduled while its predecessor runs; it waits in pdl_enter()).
+template <typename... KP, typename... A>
+static cudaError_t launch_k(bool pdl, void (*k)(KP...), dim3 g, int b, int smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = g;
+    c.blockDim = dim3((unsigned)b, 1, 1);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k, static_cast<KP>(args)...);
+}
+
+}  // namespace mg

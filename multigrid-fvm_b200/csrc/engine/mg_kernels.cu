@@ -2,7 +2,8 @@
 //
 // Three execution shapes share the per-cell arithmetic of mg_cells.cuh:
 //   * grid-wide kernels: one thread per cell, blockIdx.y selects the case, so one
-//     launch advances one routine on one level of every case in the batch;
+//     launch advances one routine on one level of every case in the batch (those that
+//     share neighbourhoods, the assembly and the transfers, by tiles: mg_tile.cu);
 //   * k_smooth: shared-memory tiles that run several smoother sweeps per launch on
 //     a tile plus a halo as deep as the sweeps (temporal blocking); it reads one
 //     buffer and writes the other, so no CTA ever loads a halo another CTA of the
@@ -16,111 +17,15 @@
 // so they are assembled in one pass and smoothed in the same launches; p' follows.
 // All reductions are two-level and fixed-order, so results are reproducible.
 #include "mg_cells.cuh"
+#include "mg_fast.cuh"
+#include "mg_grid.cuh"
 #include "mg_kernels.cuh"
+#include "mg_reduce.cuh"
 #include "mg_tangent.cuh"
 
 #include <type_traits>
 
 namespace mg {
-
-struct Dom { int i0, j0, wi, wj; };
-
-__device__ __forceinline__ Dom dom_all(const LevelDev &L) { return {0, 0, L.npx, L.npy}; }
-__device__ __forceinline__ Dom dom_interior(const LevelDev &L) { return {1, 1, L.npx - 2, L.npy - 2}; }
-__device__ __forceinline__ Dom dom_flux(const LevelDev &L) { return {0, 0, L.npx - 1, L.npy - 1}; }
-// sweep extent of each equation (solve_u/v/pprime/sc :701, :710, :725, :735)
-__device__ __forceinline__ Dom dom_eq(const LevelDev &L, int e)
-{
-    if (e == EQ_U) return {1, 1, L.npx - 3, L.npy - 2};
-    if (e == EQ_V) return {1, 1, L.npx - 2, L.npy - 3};
-    return dom_interior(L);
-}
-
-__device__ __forceinline__ bool cell_at(const Dom &d, int t, int &i, int &j)
-{
-    if (d.wi <= 0 || d.wj <= 0 || t >= d.wi * d.wj) return false;
-    j = d.j0 + t / d.wi;
-    i = d.i0 + t % d.wi;
-    return true;
-}
-
-__device__ __forceinline__ int nth_eq(int mask, int k)
-{
-    for (int e = 0; e < 4; ++e)
-        if ((mask >> e) & 1) {
-            if (k == 0) return e;
-            --k;
-        }
-    return -1;
-}
-
-// ------------------------------------------------------------ reductions
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV])
-{
-    __shared__ double red[32][NV];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    __syncthreads();
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) red[warp][k] = v[k];
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            v[k] = lane < nw ? red[lane][k] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        }
-    }
-    __syncthreads();
-}
-
-// Write this block's NV partial sums; returns true (in every thread) for the last
-// block to arrive, which then sees every block's partials.
-template <int NV>
-__device__ __forceinline__ bool publish_partials(double *partials, unsigned *counter, const double (&v)[NV],
-                                                 int nblocks)
-{
-    __shared__ int is_last;
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) partials[blockIdx.x * RED_STRIDE + k] = v[k];
-        __threadfence();
-        unsigned prev = atomicAdd(counter, 1u);
-        is_last = (prev == (unsigned)nblocks - 1u);
-    }
-    __syncthreads();
-    if (is_last) __threadfence();
-    return is_last != 0;
-}
-
-template <int NV>
-__device__ __forceinline__ void gather_partials(const double *partials, int nblocks, double (&v)[NV])
-{
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) v[k] += __ldcg(&partials[b * RED_STRIDE + k]);
-    block_sum<NV>(v);
-}
-
-// ---------------------------------------------- programmatic dependent launch
-// The V-cycle's kernels are launched with programmatic stream serialization (when the
-// schedule's `pdl` switch is on), so a kernel's CTAs may be scheduled while its
-// predecessor is still running.  Every kernel therefore starts by waiting until the
-// grids it depends on have completed and their memory is visible (a no-op for a
-// kernel launched without the attribute), and then lets its own dependent launch
-// begin: at most one kernel waits ahead of the running one, and nothing a kernel
-// reads or writes is touched before its predecessors are done.
-__device__ __forceinline__ void pdl_enter()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // ------------------------------------------------------ grid-wide kernels
 #define CASE_PROLOGUE(mode)                          \
@@ -256,83 +161,88 @@ __global__ void __launch_bounds__(BLOCK) k_asm(const CaseDev *__restrict__ cs, C
 // threads copy the ghosts of the boundary rows.
 // One interior cell of update (+ the fusions above): ppq, ppe, ppn = p' at the cell and
 // its east and north neighbours.
-// the values of its own cell an update reads besides p'
+// the values of its own cell an update reads besides p' (code: its part of the copy)
 struct UpdIn {
     double u, v, p, ax, ay, apu, apv;
+    int code;
 };
-__device__ __forceinline__ UpdIn update_in(const LevelDev &L, int q)
+template <class IO>
+__device__ __forceinline__ UpdIn update_in(const IO &io, int q, int fuse)
 {
-    return {MGF(L, S_U)[q], MGF(L, S_V)[q], MGF(L, S_P)[q], MGF(L, S_AREAX)[q], MGF(L, S_AREAY)[q],
-            MGF(L, S_APU)[q], MGF(L, S_APV)[q]};
+    return {io.ld(S_U, q), io.ld(S_V, q), io.ld(S_P, q), io.g(S_AREAX, q), io.g(S_AREAY, q), io.ld(S_APU, q),
+            io.ld(S_APV, q), (fuse & 4) && io.L.pcode ? io.L.pcode[q] : 0};
 }
-__device__ __forceinline__ void update_cell(const LevelDev &L, const CaseDev &C, int i, int j, double ppq, double ppe,
+template <class IO>
+__device__ __forceinline__ void update_cell(const IO &io, const CaseDev &C, int i, int j, double ppq, double ppe,
                                             double ppn, bool out, int fuse, const UpdIn &in)
 {
-    const int nx = L.npx, q = j * nx + i;
-    double *u = MGF(L, S_U), *v = MGF(L, S_V), *p = MGF(L, S_P);
+    const int nx = io.L.npx, q = j * nx + i;
     const double ppref = 0.0;
-    const double un = in.u + in.ax * (ppq - ppe) / in.apu;
-    const double vn = in.v + in.ay * (ppq - ppn) / in.apv;
+    const double un = in.u + quotient(in.ax * (ppq - ppe), in.apu);
+    const double vn = in.v + quotient(in.ay * (ppq - ppn), in.apv);
     const double pn = in.p + C.relxp * (ppq - ppref);
-    const int code = ((fuse & 4) && L.pcode) ? L.pcode[q] : 0;
-    if (code & ~PCODE_DST) {
-        for (int k = (code & ~PCODE_DST) - 1;; ++k) {
-            const int e = L.pfan[2 * k], src = L.pfan[2 * k + 1], dq = e & ~PFAN_END;
-            const double val = src < 0 ? pn : p[src];
-            p[dq] = val;
-            if (out && dq % nx == nx - 2) p[dq + 1] = val;
+    if (in.code & ~PCODE_DST) {
+        for (int k = (in.code & ~PCODE_DST) - 1;; ++k) {
+            const int e = io.L.pfan[2 * k], src = io.L.pfan[2 * k + 1], dq = e & ~PFAN_END;
+            const double val = src < 0 ? pn : io.ld(S_P, src);
+            io.st(S_P, dq, val);
+            if (out && dq % nx == nx - 2) io.st(S_P, dq + 1, val);
             if (e & PFAN_END) break;
         }
     }
-    const bool dst = (code & PCODE_DST) != 0;
-    if (!out || i != nx - 2) u[q] = un;
-    v[q] = vn;
-    if (!dst) p[q] = pn;
-    if (out && i == nx - 3) u[q + 1] = un;
+    const bool dst = (in.code & PCODE_DST) != 0;
+    if (out && i == nx - 2 && (fuse & 2)) io.st(S_SC, q + 1, io.ld(S_SC, q));
+    if (!out || i != nx - 2) io.st(S_U, q, un);
+    io.st(S_V, q, vn);
+    if (!dst) io.st(S_P, q, pn);
+    if (out && i == nx - 3) io.st(S_U, q + 1, un);
     if (out && i == nx - 2) {
-        v[q + 1] = vn;
-        if (!dst) p[q + 1] = pn;
-        if (fuse & 2) MGF(L, S_SC)[q + 1] = MGF(L, S_SC)[q];
+        io.st(S_V, q + 1, vn);
+        if (!dst) io.st(S_P, q + 1, pn);
     }
-}
-__device__ __forceinline__ void update_cell(const LevelDev &L, const CaseDev &C, int i, int j, double ppq, double ppe,
-                                            double ppn, bool out, int fuse)
-{
-    update_cell(L, C, i, j, ppq, ppe, ppn, out, fuse, update_in(L, j * L.npx + i));
 }
 
 // EARLY: the previous launch is a p' smoother, which writes none of the cell's other
-// operands (u, v, p, areas, apu, apv), so they are read before waiting for it (a
-// finished case, ST.done, set at the end of a cycle, loads nothing).
+// operands (u, v, p, areas, apu, apv), so they are read before waiting for it.  One round
+// trip to memory and divisions that stay on their fast path inside obstacles (quotient):
+// 86 us on level 0 of 64 256^2 cases, 112 before (57 at the measured copy rate).
 template <bool EARLY>
 __global__ void __launch_bounds__(BLOCK) k_update(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode,
                                                   int fuse)
 {
-    if (!EARLY) pdl_enter();
-    CASE_PROLOGUE(mode);
-    const Dom d = dom_interior(L);
-    const int n = d.wi * d.wj, nx = L.npx;
-    const bool out = (fuse & 1) && C.ibc_xp == 4;
+    const CaseDev &C = cs[blockIdx.y];
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
+    const int nx = L.npx, n = (nx - 2) * (L.npy - 2), t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool out = (fuse & 1) && C.ibc_xp == 4, active = mode_active(C, ig, mode);
     int i, j;
-    if (cell_at(d, t, i, j)) {
-        const int q = j * nx + i;
-        const UpdIn in = update_in(L, q);
-        if (EARLY) pdl_enter();
+    const bool cell = active && cell_at({1, 1, nx - 2, L.npy - 2}, t, i, j);
+    const int q = cell ? j * nx + i : 0;
+    UpdIn in{};
+    if (!EARLY) pdl_enter();
+    if (cell) in = update_in(io, q, fuse);
+    if (EARLY) pdl_enter();
+    if (!active) return;
+    const bool live = !st[blockIdx.y].done;
+    if (cell) {
+        double pc, pe, pn;
         if (fuse & 16) {   // mixed precision: p' is FP32, in buffer (fuse & 32 ? 1 : 0) of its correction
-            const float *pf = del32(L, EQ_PP, (fuse & 32) ? 1 : 0);
-            update_cell(L, C, i, j, (double)pf[q], (double)pf[q + 1], (double)pf[q + nx], out, fuse, in);
-            return;
+            const float *pf = reinterpret_cast<const float *>(io.at(eq_tmp(EQ_PP))) +
+                              ((fuse & 32) ? (size_t)nx * L.npy : 0) + q;
+            pc = pf[0];
+            pe = pf[1];
+            pn = pf[nx];
+        } else {
+            const double *pp = io.at((fuse & 8) ? S_TMP0 : S_PP) + q;
+            pc = pp[0];
+            pe = pp[1];
+            pn = pp[nx];
         }
-        const double *pp = MGF(L, (fuse & 8) ? S_TMP0 : S_PP);
-        const double ppq = pp[q];
-        if (fuse & 8) MGF(L, S_PP)[q] = ppq;
-        update_cell(L, C, i, j, ppq, pp[q + 1], pp[q + nx], out, fuse, in);
-    } else {
-        if (EARLY) pdl_enter();
-        if (out && t < n + 2) {
-            const int jb = t == n ? 0 : L.npy - 1;
-            row_outflow(L, jb, (fuse & 2) != 0);
-        }
+        if (!live) return;
+        update_cell(io, C, i, j, pc, pe, pn, out, fuse, in);
+        if ((fuse & (8 | 16)) == 8) io.st(S_PP, q, pc);
+    } else if (live && out && t >= n && t < n + 2) {
+        row_outflow_io(io, t == n ? 0 : L.npy - 1, (fuse & 2) != 0);
     }
 }
 
@@ -348,61 +258,44 @@ template <bool EARLY>
 __global__ void __launch_bounds__(BLOCK) k_mass_coefp(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int reduce,
                                                       int flags)
 {
-    if (!EARLY) pdl_enter();
-    CASE_PROLOGUE(mode);
-    const Dom d = dom_interior(L);
-    const int n = d.wi * d.wj, nb = (n + blockDim.x - 1) / blockDim.x;
-    if ((int)blockIdx.x >= nb) return;
-    double a[1] = {0.0};
+    const CaseDev &C = cs[blockIdx.y];
+    CaseState &ST = st[blockIdx.y];
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
+    const int n = (L.npx - 2) * (L.npy - 2), nb = (n + blockDim.x - 1) / blockDim.x;
+    const bool active = mode_active(C, ig, mode) && (int)blockIdx.x < nb;
     int i, j;
-    if (EARLY) {
-        const bool cell = cell_at(d, t, i, j);
-        Coef k;
-        double su = 0.0;
-        if (cell) mass_coefp_io(Prim{L}, C, i, j, k, su, S_U, S_V, MC_COEF);
-        pdl_enter();
-        if (cell) {
-            const Prim io{L};
-            const int q = j * L.npx + i;
-            const int us = (flags & 1) ? S_TMP0 : S_U, vs = (flags & 1) ? S_TMP1 : S_V;
-            a[0] = mass_coefp_io(io, C, i, j, k, su, us, vs, MC_SU);
+    const bool cell = active && cell_at({1, 1, L.npx - 2, L.npy - 2}, blockIdx.x * blockDim.x + threadIdx.x, i, j);
+    Coef k{};
+    double su = 0.0, a[1] = {0.0};
+    if (!EARLY) pdl_enter();
+    if (EARLY && cell) mass_coefp_io(io, C, i, j, k, su, S_U, S_V, MC_COEF);
+    if (EARLY) pdl_enter();
+    if (!active) return;
+    const bool live = !ST.done;
+    if (cell) {
+        const int q = j * L.npx + i;
+        const int us = (flags & 1) ? S_TMP0 : S_U, vs = (flags & 1) ? S_TMP1 : S_V;
+        const double u = io.ld(us, q), v = io.ld(vs, q), sc = (flags & 1) ? io.ld(S_TMP2, q) : 0.0;
+        a[0] = mass_coefp_io(io, C, i, j, k, su, us, vs, EARLY ? MC_SU : MC_ALL);
+        if (live) {
+            if ((flags & 1) && !(flags & 2)) {   // u, v, sc back from the smoother's buffers
+                if (i <= L.npx - 3) io.st(S_U, q, u);
+                if (j <= L.npy - 3) io.st(S_V, q, v);
+                io.st(S_SC, q, sc);
+            }
             if (flags & 2) {
                 const double ap = (flags & 4) ? k.ap + 1.0e-30 : k.ap;
-                op32(L, EQ_PP, CK_AW)[q] = (float)k.aw;
-                op32(L, EQ_PP, CK_AE)[q] = (float)k.ae;
-                op32(L, EQ_PP, CK_AS)[q] = (float)k.as;
-                op32(L, EQ_PP, CK_AN)[q] = (float)k.an;
-                op32(L, EQ_PP, CK_AP)[q] = (float)(1.0 / ap);
-                op32(L, EQ_PP, CK_SU)[q] = (float)su;
+                const double o[NCOEF] = {k.aw, k.ae, k.as, k.an, 1.0 / ap, su};
+#pragma unroll
+                for (int c = 0; c < NCOEF; ++c) reinterpret_cast<float *>(io.at(co_slot(EQ_PP, c)))[q] = (float)o[c];
             } else {
-                // cell_mass_coefp's stores
-                if (flags & 1) {
-                    if (i <= L.npx - 3) io.st(S_U, q, io.ld(us, q));
-                    if (j <= L.npy - 3) io.st(S_V, q, io.ld(vs, q));
-                    io.st(S_SC, q, io.ld(S_TMP2, q));
-                }
                 io.st(S_PP, q, 0.0);
                 store_coef(io, EQ_PP, q, k, su);
             }
         }
-    } else if (cell_at(d, t, i, j)) {
-        if (flags & 2) {
-            Coef k;
-            double su;
-            a[0] = mass_coefp_values(L, C, i, j, k, su, S_U, S_V);
-            const int q = j * L.npx + i;
-            const double ap = (flags & 4) ? k.ap + 1.0e-30 : k.ap;
-            op32(L, EQ_PP, CK_AW)[q] = (float)k.aw;
-            op32(L, EQ_PP, CK_AE)[q] = (float)k.ae;
-            op32(L, EQ_PP, CK_AS)[q] = (float)k.as;
-            op32(L, EQ_PP, CK_AN)[q] = (float)k.an;
-            op32(L, EQ_PP, CK_AP)[q] = (float)(1.0 / ap);
-            op32(L, EQ_PP, CK_SU)[q] = (float)su;
-        } else {
-            a[0] = cell_mass_coefp(L, C, i, j, (flags & 1) != 0);
-        }
     }
-    if (!reduce) return;
+    if (!reduce || !live) return;
     block_sum<1>(a);
     if (publish_partials<1>(C.partials, &C.counters[0], a, nb)) {
         double s[1];
@@ -940,13 +833,16 @@ __device__ __forceinline__ void pp_level_body(const CaseDev &C, CaseState &ST, c
     const double *res = (ISOLVE == MGFVM_JACOBI && (nu & 1)) ? phi2 : phi;
     const bool out = (fuse & 1) && C.ibc_xp == 4;
     // the region is the padded level (W = npx), so shared and global indices coincide
+    UpdIn inA{}, inB{};
+    if (limA >= 0) inA = update_in(Prim{L}, P.gA, fuse);
+    if (limB >= 0) inB = update_in(Prim{L}, P.gB, fuse);
     if (limA >= 0) {
         pp[P.gA] = res[kA];
-        update_cell(L, C, P.i, P.jA, res[kA], res[kA + 1], res[kA + W], out, fuse);
+        update_cell(Prim{L}, C, P.i, P.jA, res[kA], res[kA + 1], res[kA + W], out, fuse, inA);
     }
     if (limB >= 0) {
         pp[P.gB] = res[kB];
-        update_cell(L, C, P.i, P.jB, res[kB], res[kB + 1], res[kB + W], out, fuse);
+        update_cell(Prim{L}, C, P.i, P.jB, res[kB], res[kB + 1], res[kB + W], out, fuse, inB);
     }
     if (out && threadIdx.x < 2) row_outflow(L, threadIdx.x == 0 ? 0 : L.npy - 1, (fuse & 2) != 0);
     if (reduce) {
@@ -1229,13 +1125,16 @@ __device__ void band_pp(const CaseDev &C, CaseState &ST, const LevelDev &L, cons
     cluster_barrier();   // every CTA has read u, v and staged its band
     const double *res = band_units<ISOLVE>(B, d, nu, sm, stride, K);
     const bool out = (fuse & 1) && C.ibc_xp == 4;
+    UpdIn inA{}, inB{};
+    if (B.ownA) inA = update_in(Prim{L}, qA, fuse);
+    if (B.ownB) inB = update_in(Prim{L}, qB, fuse);
     if (B.ownA) {
         pp[qA] = res[K.sA];
-        update_cell(L, C, B.i, B.ja, res[K.sA], res[K.sA + 1], res[K.sA + nx], out, fuse);
+        update_cell(Prim{L}, C, B.i, B.ja, res[K.sA], res[K.sA + 1], res[K.sA + nx], out, fuse, inA);
     }
     if (B.ownB) {
         pp[qB] = res[K.sB];
-        update_cell(L, C, B.i, B.jb, res[K.sB], res[K.sB + 1], res[K.sB + nx], out, fuse);
+        update_cell(Prim{L}, C, B.i, B.jb, res[K.sB], res[K.sB + 1], res[K.sB + nx], out, fuse, inB);
     }
     if (out && B.r == 0 && threadIdx.x < 2) row_outflow(L, threadIdx.x == 0 ? 0 : L.npy - 1, (fuse & 2) != 0);
     if (reduce) {
@@ -1477,112 +1376,6 @@ __global__ void __launch_bounds__(BLOCK) k_prol_corr(const CaseDev *__restrict__
     if (cell_at(dom_interior(K), t, i, j)) cell_prol_corr(L, K, i, j);
 }
 
-template <bool FUSED>
-__global__ void __launch_bounds__(BLOCK) k_prol_apply(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode)
-{
-    pdl_enter();
-    CASE_PROLOGUE(mode);
-    const LevelDev &K = C.lv[ig + 1];
-    int i, j;
-    if (cell_at(dom_interior(L), t, i, j)) cell_prol_apply<FUSED>(L, K, i, j);
-}
-
-// End of a V-cycle on the level-0 interior: relative change of u, v, sc and of p
-// with its mean removed against the previous cycle, the history entry, the stop
-// rule, and prev <- current.  p sums are shifted by the previous cycle's means so a
-// uniform pressure drift does not cancel catastrophically.
-// The end-of-cycle work for level-0 cell index t of this block (see k_endcycle).
-// History entry and the reference's stop test (:247-248) when the fixed-point change is
-// not tracked: one thread per case.
-__device__ __forceinline__ void end_of_cycle_err_only(const CaseDev &C, CaseState &ST)
-{
-    const double err = ST.last_err;
-    const int k = ST.ncyc;
-    if (k < C.hist_cap) {
-        C.hist_err[k] = err;
-        C.hist_delta[k] = 0.0;
-    }
-    ST.ncyc = k + 1;
-    const bool finite = isfinite(err);
-    if (!finite) ST.status |= CASE_NONFINITE;
-    if (C.stop_enabled) {
-        if (!finite) ST.done = 1;
-        else if (err < C.convergence) { ST.done = 1; ST.status |= CASE_CONVERGED_REF; }
-    }
-    ST.have_prev = 0;
-}
-
-// The fixed-point change (four norms over level 0 and their block reduction) is
-// computed only while a solve with fp_tol > 0 runs; otherwise the cycle only records
-// its mass error.
-__device__ __forceinline__ void end_of_cycle(const CaseDev &C, CaseState &ST, int t, int nb)
-{
-    if (!(C.fp_tol > 0.0)) {
-        if (t == 0) end_of_cycle_err_only(C, ST);
-        return;
-    }
-    const LevelDev &L = C.lv[0];
-    const Dom d = dom_interior(L);
-    const int n = d.wi * d.wj;
-    const double kd = ST.shift_d, kp = ST.shift_p;
-    double a[10];
-#pragma unroll
-    for (int k = 0; k < 10; ++k) a[k] = 0.0;
-    int i, j;
-    if (cell_at(d, t, i, j)) {
-        const int q = j * L.npx + i;
-        const int cur[3] = {S_U, S_V, S_SC}, prv[3] = {S_PREV_U, S_PREV_V, S_PREV_SC};
-#pragma unroll
-        for (int f = 0; f < 3; ++f) {
-            double x = MGF(L, cur[f])[q], y = MGF(L, prv[f])[q], dd = x - y;
-            a[2 * f] = dd * dd;
-            a[2 * f + 1] = x * x;
-            MGF(L, prv[f])[q] = x;
-        }
-        double x = MGF(L, S_P)[q], y = MGF(L, S_PREV_P)[q];
-        double dd = (x - y) - kd, e = x - kp;
-        a[6] = dd; a[7] = dd * dd; a[8] = e; a[9] = e * e;
-        MGF(L, S_PREV_P)[q] = x;
-    }
-    block_sum<10>(a);
-    if (!publish_partials<10>(C.partials, &C.counters[1], a, nb)) return;
-    double s[10];
-    gather_partials<10>(C.partials, nb, s);
-    if (threadIdx.x != 0) return;
-    C.counters[1] = 0;
-    const double N = (double)n;
-    double worst = 0.0;
-    for (int f = 0; f < 4; ++f) {
-        double num, den;
-        if (f < 3) { num = s[2 * f]; den = s[2 * f + 1]; }
-        else {
-            num = s[7] - s[6] * s[6] / N;
-            den = s[9] - s[8] * s[8] / N;
-            if (num < 0.0) num = 0.0;
-        }
-        double r = num == 0.0 ? 0.0 : (den <= 0.0 ? (double)INFINITY : sqrt(num / den));
-        if (r > worst || r != r) worst = r;
-    }
-    const double err = ST.last_err;
-    const int k = ST.ncyc;
-    const double delta = ST.have_prev ? worst : 0.0;
-    if (k < C.hist_cap) {
-        C.hist_err[k] = err;
-        C.hist_delta[k] = delta;
-    }
-    ST.ncyc = k + 1;
-    ST.shift_d = kd + s[6] / N;
-    ST.shift_p = kp + s[8] / N;
-    const bool finite = isfinite(err) && isfinite(delta);
-    if (!finite) ST.status |= CASE_NONFINITE;
-    if (C.stop_enabled) {
-        if (!finite) ST.done = 1;
-        else if (err < C.convergence) { ST.done = 1; ST.status |= CASE_CONVERGED_REF; }
-        else if (C.fp_tol > 0.0 && ST.have_prev && delta < C.fp_tol) { ST.done = 1; ST.status |= CASE_CONVERGED_FP; }
-    }
-    ST.have_prev = 1;
-}
-
 __global__ void __launch_bounds__(BLOCK) k_endcycle(const CaseDev *__restrict__ cs, CaseState *st)
 {
     pdl_enter();
@@ -1592,23 +1385,9 @@ __global__ void __launch_bounds__(BLOCK) k_endcycle(const CaseDev *__restrict__ 
     const Dom d = dom_interior(C.lv[0]);
     const int n = d.wi * d.wj, nb = (n + blockDim.x - 1) / blockDim.x;
     if ((int)blockIdx.x >= nb) return;
-    end_of_cycle(C, ST, blockIdx.x * blockDim.x + threadIdx.x, nb);
-}
-
-// prolongation into level 0 followed by the end of the cycle: every thread reads
-// back only the level-0 cell it just wrote.
-template <bool FUSED>
-__global__ void __launch_bounds__(BLOCK) k_prol_apply_end(const CaseDev *__restrict__ cs, CaseState *st, int mode)
-{
-    pdl_enter();
-    const int ig = 0;
-    CASE_PROLOGUE(mode);
-    const Dom d = dom_interior(L);
-    const int n = d.wi * d.wj, nb = (n + blockDim.x - 1) / blockDim.x;
-    if ((int)blockIdx.x >= nb) return;
     int i, j;
-    if (cell_at(d, t, i, j)) cell_prol_apply<FUSED>(L, C.lv[1], i, j);
-    end_of_cycle(C, ST, t, nb);
+    const bool cell = cell_at(d, blockIdx.x * blockDim.x + threadIdx.x, i, j);
+    end_of_cycle(C, ST, cell, i, j, nb);
 }
 
 // ------------------------------------------------- one-CTA coarse kernel
@@ -1955,24 +1734,6 @@ cudaError_t configure_kernels()
     return e;
 }
 
-// Launch `k` on `st`, with programmatic stream serialization when `pdl` (the kernel
-// may then be scheduled while its predecessor runs; it waits in pdl_enter()).
-template <typename... KP, typename... A>
-static cudaError_t launch_k(bool pdl, void (*k)(KP...), dim3 g, int b, int smem, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = g;
-    c.blockDim = dim3((unsigned)b, 1, 1);
-    c.dynamicSmemBytes = (size_t)smem;
-    c.stream = st;
-    c.attrs = at;
-    c.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&c, k, static_cast<KP>(args)...);
-}
-
 // launch_k for a kernel whose CTAs form clusters of `cx` along x
 template <typename... KP, typename... A>
 static cudaError_t launch_cluster(bool pdl, void (*k)(KP...), dim3 g, int b, int smem, cudaStream_t st, int cx,
@@ -2055,7 +1816,8 @@ cudaError_t launch_one(const Launch &X, const CaseDev *dc, CaseState *ds, const 
     switch (X.kernel) {
     case K_FLUXES: le = launch_k(pdl, k_fluxes, g, b, 0, st, dc, ds, X.ig, X.mode); break;
     case K_ASM:
-        if (X.a1) le = launch_k(pdl, k_asm<1>, g, b, 0, st, dc, ds, X.ig, X.mode, (unsigned)X.a0);
+        if (X.a1 == 2) le = launch_tile(X, dc, ds, S, st);
+        else if (X.a1) le = launch_k(pdl, k_asm<1>, g, b, 0, st, dc, ds, X.ig, X.mode, (unsigned)X.a0);
         else le = launch_k(pdl, k_asm<0>, g, b, 0, st, dc, ds, X.ig, X.mode, (unsigned)X.a0);
         break;
     case K_MASS_COEFP:
@@ -2120,23 +1882,21 @@ cudaError_t launch_one(const Launch &X, const CaseDev *dc, CaseState *ds, const 
             le = launch_cluster(pdl, k_band_visit<MGFVM_GAUSS_SEIDEL>, g, b, X.smem, st, (int)g.x, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2, X.a3, X.a4);
         break;
     case K_PFIX_BOUND: le = launch_k(pdl, k_pfix_bound, g, b, 0, st, dc, ds, X.ig, X.mode, X.a0); break;
-    case K_RESTV_FLUXES: le = launch_k(pdl, k_restv_fluxes, g, b, 0, st, dc, ds, X.ig, X.mode); break;
-    case K_RESTRICT: le = launch_k(pdl, k_restrict, g, b, 0, st, dc, ds, X.ig, X.mode, (unsigned)X.a0); break;
+    case K_RESTV_FLUXES:
+        if (X.a1 == 2) le = launch_tile(X, dc, ds, S, st);
+        else le = launch_k(pdl, k_restv_fluxes, g, b, 0, st, dc, ds, X.ig, X.mode); break;
+    case K_RESTRICT:
+        if (X.a1 == 2) le = launch_tile(X, dc, ds, S, st);
+        else le = launch_k(pdl, k_restrict, g, b, 0, st, dc, ds, X.ig, X.mode, (unsigned)X.a0); break;
     case K_PROL_CORR: le = launch_k(pdl, k_prol_corr, g, b, 0, st, dc, ds, X.ig, X.mode); break;
     case K_PROL_APPLY:
-        if (X.a0) le = launch_k(pdl, k_prol_apply<true>, g, b, 0, st, dc, ds, X.ig, X.mode);
-        else le = launch_k(pdl, k_prol_apply<false>, g, b, 0, st, dc, ds, X.ig, X.mode);
-        break;
+    case K_PROL_APPLY_END: le = launch_tile(X, dc, ds, S, st); break;
     case K_TAIL: le = launch_k(pdl, k_tail, g, b, X.smem, st, dc, ds, S, X.smem / (int)sizeof(double)); break;
     case K_TAIL_TAN:
         if (!dt) return cudaErrorInvalidValue;
         le = launch_k(pdl, k_tail_tan, g, b, 0, st, dc, ds, dt, S);
         break;
     case K_ENDCYCLE: le = launch_k(pdl, k_endcycle, g, b, 0, st, dc, ds); break;
-    case K_PROL_APPLY_END:
-        if (X.a0) le = launch_k(pdl, k_prol_apply_end<true>, g, b, 0, st, dc, ds, X.mode);
-        else le = launch_k(pdl, k_prol_apply_end<false>, g, b, 0, st, dc, ds, X.mode);
-        break;
     default: return cudaErrorInvalidValue;
     }
     return le != cudaSuccess ? le : cudaGetLastError();

@@ -10,15 +10,15 @@ namespace mg {
 // One kernel launch of a V-cycle (or single-op) schedule.
 enum KernelId {
     K_FLUXES = 0,    // fluxes only (single-op)
-    K_ASM,           // fused assembly: a0 = AsmBits, a1 = 1: fluxes recomputed live
+    K_ASM,           // fused assembly: a0 = AsmBits, a1 = 1: fluxes recomputed live, 2: by tiles
     K_MASS_COEFP,    // a0 = reduce the mass error into CaseDev::last_err
     K_UPDATE,
     K_PFIX,          // a0 = phase (0 gather, 1 scatter, 2 both)
     K_BOUND,         // a0 = bits: 1 periodic, 2 outflow u/v/p, 4 outflow sc
     K_SMOOTH,        // tile smoother: a0 = eq mask, a1 = first unit, a2 = units, a3 = dir, a4 = tile
     K_COPY,          // copy equations' buffers back: a0 = eq mask
-    K_RESTV_FLUXES,  // restv + fine fluxes
-    K_RESTRICT,      // restr{u,v,sc} + coarse fluxes
+    K_RESTV_FLUXES,  // restv + fine fluxes + fine residuals (a1 = 2: by tiles, their sums)
+    K_RESTRICT,      // restr{u,v,sc} + coarse fluxes, a0 = AsmBits (a1 = 2: by tiles)
     K_PROL_CORR, K_PROL_APPLY,   // prol_apply: a0 = 1 forms the corrections itself (no K_PROL_CORR before it)
     K_TAIL, K_ENDCYCLE, K_PROL_APPLY_END,
     K_SMOOTH_F32,    // mixed precision: the tiles of K_SMOOTH on FP32 operands and corrections
@@ -97,6 +97,8 @@ struct CaseTan;
 cudaError_t launch_one(const Launch &L, const CaseDev *dcases, CaseState *dstate, const CaseTan *dtan,
                        const Sched &S, cudaStream_t stream);
 cudaError_t configure_kernels();
+// the tile kernels (mg_tile.cu)
+cudaError_t launch_tile(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
 
 // Kernels of the raw-pointer entry points.
 cudaError_t raw_jacobi(const double *aw, const double *ae, const double *as, const double *an,
