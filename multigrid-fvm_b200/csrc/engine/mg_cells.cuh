@@ -403,21 +403,19 @@ __device__ __forceinline__ T gs_value(const T &aw, const T &ae, const T &as, con
 // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., sec. 4.7):
 // q0 = RN(a y); r0 = a - b q0 and q1 = RN(q0 + r0 y) make q1 faithful (|q1 - a/b| <
 // ulp), so r1 = a - b q1 is exact and q2 = RN(q1 + r1 y) = RN(a/b).  The theorem needs
-// no underflow or overflow anywhere: operands outside [2^-450, 2^450) in magnitude
-// (which keeps the quotient within [2^-900, 2^900]), zero divisors, Inf and NaN take the
-// IEEE division, except the two dividends that fill the inside of obstacles, where the
-// 1e30 diagonals drive values down by 1e-30 a cell: a zero's quotient is q0, whose sign is
-// the division's, and a tiny one is divided after scaling by 2^600 (exact) and scaled back,
-// exact where the quotient is normal and a correctly signed zero where it is below half the
-// smallest subnormal; only subnormal quotients are left to the IEEE division.  Results are
-// therefore the bits of a / b in every case.  (The compiled IEEE division takes a slow path
-// for such dividends.)  The ranges are tested on the high words, off the FP64 pipe; a recip with y = 0 stands for
-// a divisor out of range.
+// no underflow or overflow anywhere.  That holds for |b| in [2^-450, 2^102) and |a| in
+// [2^-918, 2^450): quotients are normal and below 2^900, and the remainders, multiples of
+// ulp(q) ulp(b) > |a| 2^-106 >= 2^-1024, are representable.  Every other divisor (a recip
+// with y = 0) and dividend goes through div_by_rare, so results are the bits of a / b in
+// every case.  The dividend's range reaches this far down because the 1e30 diagonals inside
+// obstacles drive values down by 1e-30 a cell: with a bound of 2^-450 one cell in a hundred
+// of a 256^2 obstacle case left it, and the warps holding those paced every barrier.
+// The ranges are tested on the high words, off the FP64 pipe.
 struct Recip {
     double b, y;
 };
 
-// |x| in [2^lo, 2^hi)
+// |x| in [2^LO, 2^HI)
 template <int LO, int HI>
 __device__ __forceinline__ bool exponent_in(double x)
 {
@@ -427,7 +425,7 @@ __device__ __forceinline__ bool exponent_in(double x)
 __device__ __forceinline__ Recip make_recip(double b)
 {
     const double y = 1.0 / b;
-    return {b, exponent_in<-450, 450>(b) ? y : 0.0};
+    return {b, exponent_in<-450, 102>(b) ? y : 0.0};
 }
 
 __device__ __forceinline__ double markstein(double a, const Recip &R)
@@ -439,13 +437,23 @@ __device__ __forceinline__ double markstein(double a, const Recip &R)
     return fma(r1, R.y, q1);
 }
 
-// div_by's operands outside the plain range (a call: inlined at every division it would
-// crowd the instruction cache)
+// markstein's steps give the quotient
+__device__ __forceinline__ bool div_plain(double a, const Recip &R)
+{
+    return exponent_in<-918, 450>(a) & (__double2hiint(R.y) != 0);
+}
+
+// a / b outside that (a call: inlined at every division it would crowd the instruction
+// cache).  The compiled division takes a slow path for the dividends met here in earnest,
+// zeros (fields at rest) and tiny ones: a zero's quotient is q0, whose sign is the
+// division's, and a tiny one is divided after scaling by 2^600 (exact) and scaled back,
+// exact where the quotient is normal and a correctly signed zero where it is below half the
+// smallest subnormal.
 static __device__ __noinline__ double div_by_rare(double a, double b, double y)
 {
     if (__double2hiint(y) != 0) {
         if (a == 0.0) return a * y;
-        if (fabs(a) < 0x1p-450) {
+        if (fabs(a) < 0x1p-918) {
             const double q = markstein(a * 0x1p600, Recip{b, y});
             if (exponent_in<-422, 1023>(q) || fabs(q) < 0x1p-476) return q * 0x1p-600;
         }
@@ -455,7 +463,7 @@ static __device__ __noinline__ double div_by_rare(double a, double b, double y)
 
 __device__ __forceinline__ double div_by(double a, const Recip &R)
 {
-    if (exponent_in<-450, 450>(a) && __double2hiint(R.y) != 0) return markstein(a, R);
+    if (div_plain(a, R)) return markstein(a, R);
     return div_by_rare(a, R.b, R.y);
 }
 

@@ -46,6 +46,7 @@ using namespace mg;
 static_assert(PFAN_LAST == mg::PFAN_END, "fan-list end marker differs between host and device");
 static const int TAIL_AUTO_CELLS = 0;   // automatic choice: grid kernels on every level (measured fastest)
 static const int HIST_INITIAL = 4096;
+static const int SMS = 148;
 
 struct mgfvm_ctx {
     int device = 0;
@@ -110,7 +111,7 @@ static inline int nblk(long long n) { return (int)std::max<long long>(1, (n + BL
 static double recip_of(double b)
 {
     const double m = std::fabs(b);
-    return m >= 0x1p-450 && m < 0x1p450 ? 1.0 / b : 0.0;
+    return m >= 0x1p-450 && m < 0x1p102 ? 1.0 / b : 0.0;
 }
 
 // ------------------------------------------------------------------ schedule
@@ -280,7 +281,7 @@ struct Builder {
     }
     // Whether the visits to level ig run as band visits (k_band_visit, FP64 in either
     // precision): the level fits a cluster and the tuning asks for them, or leaves it
-    // to the default, which takes them for batches of at least BAND_MIN_CASES cases
+    // to the default, which takes them for large batches (band_default) of cases
     // that all have the level at one size (a launch is shaped for its largest case, so
     // smaller ones would leave most of their clusters' threads idle).
     bool band_visits(int ig, int mode, int &G, int &blk, int &smem) const
@@ -290,7 +291,16 @@ struct Builder {
         return mode != M_OP && x->sched.nswpp > 0 && t != 1 &&
                (isolve == MGFVM_JACOBI || isolve == MGFVM_GAUSS_SEIDEL) && !whole_level(ig, mx, my) &&
                band_level(ig, G, blk, smem) &&
-               (t == 2 || (x->ncases >= BAND_MIN_CASES && one_size(ig, mx, my)));
+               (t == 2 || (band_default(G) && one_size(ig, mx, my)));
+    }
+    // The sizes of batch at which band visits of a G-CTA level are the faster ones.  FP64:
+    // only where a pair of CTAs holds the level (66^2 of a 256^2 case; 64 cases 2.59 ms per
+    // V-cycle against 2.64 with tiles, 32 cases 1.40 against 1.36; on 130^2 they cost 2.75).
+    // Mixed precision, whose tiles are FP32 and slower here: BAND_MIN_CASES.
+    bool band_default(int G) const
+    {
+        if (x->opt.precision == MGFVM_PREC_MIXED) return x->ncases >= BAND_MIN_CASES;
+        return G <= 2 && x->ncases >= 2 * BAND_MIN_CASES;
     }
     // every case that has level ig has it at mx x my
     bool one_size(int ig, int mx, int my) const
@@ -298,6 +308,61 @@ struct Builder {
         for (const mgfvm_config &c : x->cfg)
             if (ig < c.ngrid && (npx_of(c, ig) != mx || npy_of(c, ig) != my)) return false;
         return true;
+    }
+    // The register-blocked smoother's plan for `units` units of `neq` equations on level ig:
+    // launches, tile and tiles per case; false where k_smooth's tiles are expected to be
+    // faster, or the tuning asks for those.  Expected times in microseconds, fitted to both
+    // kernels on 1 to 64 cases of 64^2 to 1024^2: a round of CTAs over the SMs takes 4.9 +
+    // 0.37 a unit here and 5.0 + 0.19 there; the tiles here are larger, so large levels need
+    // half as many rounds, while a level of one round either way favours k_smooth's faster
+    // units unless a single launch can take all of them.  (p' on two cases, 20 units: 256^2
+    // 19.0 against 28.8 us, 128^2 17.7 against 14.4, 64^2 13.2 in one launch against 14.4.)
+    struct QPlan {
+        int chunks, tw, th, tiles;
+    };
+    bool smooth_q_plan(int ig, int neq, int units, bool tmp_ok, QPlan &best) const
+    {
+        if (x->sched.isolve != MGFVM_GAUSS_SEIDEL || x->tune.smooth_threads[ig] || x->tune.smooth_units[ig] ||
+            x->tune.smooth_tma[ig] == 2)
+            return false;
+        int wi = 0, wj = 0;
+        for (const mgfvm_config &c : x->cfg)
+            if (ig < c.ngrid) {
+                wi = std::max(wi, npx_of(c, ig) - 2);
+                wj = std::max(wj, npy_of(c, ig) - 2);
+            }
+        // rounds of CTAs of tw x th tiles over the SMs, and the tiles of the largest case
+        auto rounds = [&](int tw, int th, int &tiles) {
+            long long n = 0;
+            tiles = 1;
+            for (const mgfvm_config &c : x->cfg)
+                if (ig < c.ngrid) {
+                    const int t = ((npx_of(c, ig) - 2 + tw - 1) / tw) * ((npy_of(c, ig) - 2 + th - 1) / th);
+                    tiles = std::max(tiles, t);
+                    n += (long long)t * neq;
+                }
+            return (double)((n + SMS - 1) / SMS);
+        };
+        auto side = [](int n, int most) { return (n + (n + most - 1) / most - 1) / ((n + most - 1) / most); };
+        double t_best = 1e300, t_old = 1e300;
+        int dummy;
+        for (int c = 1; c <= units; ++c) {
+            if ((c & 1) && !tmp_ok && c < units) continue;      // an odd count needs a copy back
+            const int u = (units + c - 1) / c;
+            const int mx = SMOOTH_Q_COLS - 2 * u - 1, my = SMOOTH_Q_ROWS - 2 * u - 1;
+            if (mx >= MIN_TILE && my >= MIN_TILE) {
+                QPlan p{c, side(wi, mx), side(wj, my), 0};
+                const double t = c * (0.3 + rounds(p.tw, p.th, p.tiles) * (4.9 + 0.37 * u));
+                if (t < t_best) {
+                    t_best = t;
+                    best = p;
+                }
+            }
+            const int tile = smooth_pairs_side(u, SMOOTH_BLOCK);
+            if (u <= MAX_UNITS && c <= (units + MAX_UNITS - 1) / MAX_UNITS + 1)
+                t_old = std::min(t_old, c * (0.3 + rounds(tile, tile, dummy) * (5.0 + 0.19 * u)));
+        }
+        return t_best < t_old;
     }
     int f32_buf = 0;   // the FP32 correction buffer the last F32 smoothing call ended in
     bool smooth(int ig, int mode, int mask, int nsw, bool tmp_ok = false)
@@ -343,6 +408,24 @@ struct Builder {
             L.grid = dim3(1, x->ncases, neq);
             L.block = round32(mx * ((my + 1) / 2));
             L.smem = smem_for(mx * my);
+            return false;
+        }
+        QPlan qp;
+        if (smooth_q_plan(ig, neq, units, tmp_ok, qp)) {
+            int u0 = 0;
+            for (int c = 0; c < qp.chunks; ++c) {
+                const int nu = units / qp.chunks + (c < units % qp.chunks ? 1 : 0);
+                // a later launch reads its coefficients before waiting for the one before it
+                Launch &L = add(K_SMOOTH_Q, ig, mode, 0, mask, u0, nu, (c & 1) | (c > 0 && x->sched.pdl ? 4 : 0));
+                L.bw = qp.tw;
+                L.bh = qp.th;
+                L.grid = dim3((unsigned)qp.tiles, x->ncases, neq);
+                L.block = SMOOTH_Q_THREADS;
+                u0 += nu;
+            }
+            if ((qp.chunks & 1) == 0) return false;
+            if (tmp_ok) return true;
+            add(K_COPY, ig, mode, cells(ig), mask).grid.z = neq;
             return false;
         }
         const int tt = x->tune.smooth_threads[ig];
@@ -432,7 +515,7 @@ struct Builder {
     {
         if (!x->sched.pdl || mode == M_OP || out->empty()) return false;
         const int k = out->back().kernel;
-        return k == K_SMOOTH || k == K_SMOOTH_F32 || k == K_SMOOTH_TMA || k == K_COPY;
+        return k == K_SMOOTH || k == K_SMOOTH_F32 || k == K_SMOOTH_TMA || k == K_SMOOTH_Q || k == K_COPY;
     }
     // returns the update's fuse bits (0: outflow still to do)
     // `bound_bits` != 0: pbound/outflow follow the obstacle pressure copy (k_bound bits);

@@ -1847,6 +1847,7 @@ cudaError_t launch_one(const Launch &X, const CaseDev *dc, CaseState *ds, const 
             else le = launch_smooth_f32<MGFVM_GAUSS_SEIDEL, false>(pdl, X, g, b, dc, ds, st);
         }
         break;
+    case K_SMOOTH_Q: le = launch_smooth_q(X, dc, ds, S, st); break;
     case K_COPY: le = launch_k(pdl, k_copy, g, b, 0, st, dc, ds, X.ig, X.mode, X.a0); break;
     case K_SMOOTH_TMA:
         if (b > SMOOTH_BLOCK || !X.ptr || X.smem > SMOOTH_TMA_SMEM_MAX || (X.bw & 1)) return cudaErrorInvalidValue;

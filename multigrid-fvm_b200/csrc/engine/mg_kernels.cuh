@@ -36,6 +36,8 @@ enum KernelId {
     K_COARSE_CYCLE,  // the V-cycle from the restriction into level a0 (every level from a0
                      // one CTA holds) to the prolongation out of it, a cluster of 3 CTAs per
                      // case: a1 = p' units, a2 = u/v/sc units
+    K_SMOOTH_Q,      // register-blocked tile smoother (mg_smooth.cu): K_SMOOTH's a0-a3,
+                     // bw x bh = tile
     K_NKERNELS
 };
 
@@ -76,10 +78,10 @@ constexpr int SMOOTH_BLOCK = 1024;
 // dynamic shared memory per CTA (the band and its two halo rows, two buffers for Jacobi)
 constexpr int BAND_MAX_CTAS = 8;
 constexpr int BAND_SMEM_MAX = 80 * 1024;
-// By default a level runs band visits in batches of at least this many cases (of one
-// size at that level): a unit costs about a microsecond there (its cluster barrier),
-// which only pays when the tile launches it replaces have enough work to be slow too
-// (256^2 cases, levels 1-2: slower up to 16 cases, faster from 32)
+// By default a mixed-precision context runs band visits in batches of at least this many
+// cases (of one size at the level), an FP64 one in larger ones (band_default): a unit costs
+// about a microsecond there (its cluster barrier), which only pays when the tile launches it
+// replaces have enough work to be slow too
 constexpr int BAND_MIN_CASES = 32;
 // interior rows of each band when G CTAs share a level of npy padded rows (even; the
 // last band may be shorter)
@@ -99,6 +101,11 @@ cudaError_t launch_one(const Launch &L, const CaseDev *dcases, CaseState *dstate
 cudaError_t configure_kernels();
 // the tile kernels (mg_tile.cu)
 cudaError_t launch_tile(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
+
+// The register-blocked smoother (mg_smooth.cu): the region its CTA holds, a thread for
+// every 2 x 4 cells, 12 warps: three on each partition of an SM, 168 registers a thread.
+constexpr int SMOOTH_Q_COLS = 54, SMOOTH_Q_ROWS = 56, SMOOTH_Q_THREADS = 384;
+cudaError_t launch_smooth_q(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
 
 // Kernels of the raw-pointer entry points.
 cudaError_t raw_jacobi(const double *aw, const double *ae, const double *as, const double *an,
