@@ -148,9 +148,18 @@ __device__ __forceinline__ void case_barrier()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Every cell of a phase, spread over the case's cluster.
+// This worker's first index in a phase whose group has handed out `base` indices before it:
+// the phases of a group share the workers as if their cells were one list.
+__device__ __forceinline__ int wk_from(int base)
+{
+    const int t = wk_id() - base % wk_n();
+    return t < 0 ? t + wk_n() : t;
+}
+
+// Every cell of a phase, spread over the case's cluster; `base` as wk_from, advanced by the
+// phase's indices.
 template <class Fn>
-__device__ __forceinline__ void phase_cells(const CaseDev &C, const Phase &P, Fn f)
+__device__ __forceinline__ void phase_cells(const CaseDev &C, const Phase &P, int &base, Fn f)
 {
     const LevelDev &L = C.lv[P.ig];
     const LevelDev *K = P.ig + 1 < C.ngrid ? &C.lv[P.ig + 1] : nullptr;
@@ -159,19 +168,21 @@ __device__ __forceinline__ void phase_cells(const CaseDev &C, const Phase &P, Fn
     if (P.kind == P_GS) {
         // cells of colour b: (i + j) & 1 == b
         const int wr = (d.wi + 1) >> 1, n = wr * d.wj;
-        for (int t = wk_id(); t < n; t += wk_n()) {
+        for (int t = wk_from(base); t < n; t += wk_n()) {
             const int j = d.j0 + t / wr;
             const int i = d.i0 + (((d.i0 + j) & 1) != P.b ? 1 : 0) + 2 * (t % wr);
             if (i <= d.i0 + d.wi - 1) f(i, j);
         }
+        base += n;
         return;
     }
     const int n = d.wi * d.wj;
-    for (int t = wk_id(); t < n; t += wk_n()) {
+    for (int t = wk_from(base); t < n; t += wk_n()) {
         const int i = d.i0 + t % d.wi, j = d.j0 + t / d.wi;
         if (P.kind == P_JAC_RING && i != d.i0 && i != d.i0 + d.wi - 1 && j != d.j0 && j != d.j0 + d.wj - 1) continue;
         f(i, j);
     }
+    base += n;
 }
 
 // ------------------------------------------------------- forward (taped)
@@ -243,6 +254,63 @@ __device__ void tape_copy(const CaseDev &C, const CaseAdj &A, const Phase &P, bo
             for (int k = wk_id(); k < L.ncopy; k += wk_n()) t[k] = L.pbuf[k];
         else
             for (int k = wk_id(); k < L.ncopy; k += wk_n()) L.pbuf[k] = t[k];
+    }
+}
+
+// What phase P overwrites when it runs at (i, j), between the level and the tape (save: to
+// the tape).  Every phase writes at places that belong to the visited cell alone (its own
+// index on the written level; a row's outlet ghosts; a copy's destination), and no cell
+// reads what another cell of its group writes, so each thread saves or restores in the pass
+// that runs or transposes the cell, without a barrier between the two.
+__device__ __forceinline__ void tape_cell(const CaseDev &C, const CaseAdj &A, const Phase &P, int i, int j, bool save)
+{
+    const LevelDev &L = C.lv[write_level(P)];
+    const int q = j * L.npx + i;
+    const long long n = (long long)L.npx * L.npy;
+    double *t = A.tape + P.off;
+    auto keep = [&](double *a, int at, int k) {
+        if (save) t[k] = a[at];
+        else a[at] = t[k];
+    };
+    auto own = [&](int slot, int k) { keep(L.f[slot] + q, 0, (int)(k * n + q)); };
+    switch (P.kind) {
+    case P_ASM_U: case P_ASM_V: case P_ASM_SC: {
+        const int e = P.kind == P_ASM_U ? EQ_U : P.kind == P_ASM_V ? EQ_V : EQ_SC;
+        for (int c = 0; c < NCOEF; ++c) own(co_slot(e, c), c);
+        if (e != EQ_SC) own(e == EQ_U ? S_APU : S_APV, NCOEF);
+        break;
+    }
+    case P_SC_OUTFLOW: own(S_SC, 0); break;
+    case P_JAC_RING: own(tmp_of(P.a), 0); break;
+    case P_JAC_SWEEP: own(P.b == 0 ? tmp_of(P.a) : field_of(P.a), 0); break;
+    case P_JAC_COPY: own(field_of(P.a), 0); break;
+    case P_MASS_COEFP:
+        if (P.a & MC_COEF) {
+            for (int c = 0; c < NCOEF - 1; ++c) own(co_slot(EQ_PP, c), c);
+            own(S_PP, NCOEF - 1);
+        }
+        if (P.a & MC_SU) own(co_slot(EQ_PP, CK_SU), (P.a & MC_COEF) ? NCOEF : 0);
+        break;
+    case P_UPDATE: own(P.a == 1 ? S_U : P.a == 2 ? S_V : S_P, 0); break;
+    case P_PFIX: case P_PFIX_SCATTER: keep(L.f[S_P], L.pdst[i], i); break;
+    case P_PFIX_GATHER: keep(L.pbuf, i, i); break;
+    case P_OUTFLOW: {
+        const int g = j * L.npx + L.npx - 1;
+        keep(L.f[S_U], g - 1, j);
+        keep(L.f[S_V], g, L.npy + j);
+        keep(L.f[S_P], g, 2 * L.npy + j);
+        if (P.b) keep(L.f[S_SC], g, 3 * L.npy + j);
+        break;
+    }
+    case P_RESTV:
+        own(P.a == 1 ? S_U : P.a == 2 ? S_V : P.a == 4 ? S_P : S_SC, 0);
+        own(P.a == 1 ? S_RU : P.a == 2 ? S_RV : P.a == 4 ? S_RP : S_RSC, 1);
+        break;
+    case P_FINE_RES: own(tmp_of(res_eq(P.a)), 0); break;
+    case P_RESTRICT: own(P.a == 0 ? S_RESU : P.a == 1 ? S_RESV : S_RESSC, 0); break;
+    case P_PROL_CORR: own(P.a == 1 ? S_CU : P.a == 2 ? S_CV : P.a == 4 ? S_CP : S_C, 0); break;
+    case P_PROL_APPLY: own(P.a == 1 ? S_U : P.a == 2 ? S_V : P.a == 4 ? S_P : S_SC, 0); break;
+    default: break;
     }
 }
 
@@ -374,26 +442,31 @@ __device__ __forceinline__ void adj_cell(const CaseDev &C, const CaseTan &B, con
 
 // The cells of a half-sweep phase with their index in its colour-only tape.
 template <class Fn>
-__device__ __forceinline__ void gs_cells(const LevelDev &L, const Phase &P, Fn f)
+__device__ __forceinline__ void gs_cells(const LevelDev &L, const Phase &P, int &base, Fn f)
 {
     const Box d = box_eq(L.npx, L.npy, P.a);
     if (d.wi <= 0 || d.wj <= 0) return;
     const int wr = (d.wi + 1) >> 1, n = wr * d.wj;
-    for (int t = wk_id(); t < n; t += wk_n()) {
+    for (int t = wk_from(base); t < n; t += wk_n()) {
         const int j = d.j0 + t / wr;
         const int i = d.i0 + (((d.i0 + j) & 1) != P.b ? 1 : 0) + 2 * (t % wr);
         if (i <= d.i0 + d.wi - 1) f(i, j, t);
     }
+    base += n;
 }
 
 // A half-sweep, taped, in one pass: each cell's old value to the tape, then its update
 // (its neighbours are of the other colour, which the half-sweep does not write).
 __device__ __forceinline__ void fwd_gs_cell(const LevelDev &L, int e, int i, int j, double *tape, int t)
 {
-    const int q = j * L.npx + i;
-    double *f = L.f[field_of(e)];
-    tape[t] = f[q];
-    cell_gs_io(Prim{L}, e, field_of(e), q);
+    const int nx = L.npx, q = j * nx + i;
+    double *f = L.f[field_of(e)] + q;
+    const double old = f[0];
+    const double z = gs_value(L.f[co_slot(e, CK_AW)][q], L.f[co_slot(e, CK_AE)][q], L.f[co_slot(e, CK_AS)][q],
+                              L.f[co_slot(e, CK_AN)][q], L.f[co_slot(e, CK_AP)][q], L.f[co_slot(e, CK_SU)][q], f[-1],
+                              f[1], f[-nx], f[nx]);
+    tape[t] = old;
+    f[0] = z;
 }
 
 // The transpose of one red-black half-sweep cell, phi_c = (sum a_nb phi_nb + su) / ap
@@ -407,29 +480,30 @@ __device__ __forceinline__ void fwd_gs_cell(const LevelDev &L, int e, int i, int
 __device__ __forceinline__ void adj_gs_cell(const LevelDev &L, const LevelTan &B, int e, int i, int j,
                                             const double *tape, int t)
 {
+    // every load before the first store, which they could not be moved above
     const int nx = L.npx, q = j * nx + i, phi = field_of(e);
-    double *f = L.f[phi];
-    const double val = f[q];
-    f[q] = tape[t];
-    double *yp = B.t[phi] + q;
-    const double yb = *yp;
-    *yp = 0.0;
+    double *f = L.f[phi] + q, *b = B.t[phi] + q;
+    const double val = f[0], old = tape[t], yb = b[0];
+    const double pw = f[-1], pe = f[1], ps = f[-nx], pn = f[nx];
+    double k[NCOEF - 1], bk[NCOEF];
+#pragma unroll
+    for (int c = 0; c < NCOEF - 1; ++c) k[c] = L.f[co_slot(e, c)][q];
+#pragma unroll
+    for (int c = 0; c < NCOEF; ++c) bk[c] = B.t[co_slot(e, c)][q];
+    f[0] = old;
     if (yb == 0.0) return;
-    const double aw = L.f[co_slot(e, CK_AW)][q], ae = L.f[co_slot(e, CK_AE)][q], as = L.f[co_slot(e, CK_AS)][q],
-                 an = L.f[co_slot(e, CK_AN)][q], ap = L.f[co_slot(e, CK_AP)][q];
-    const double pw = f[q - 1], pe = f[q + 1], ps = f[q - nx], pn = f[q + nx];
-    const double ya = yb / ap;
-    B.t[co_slot(e, CK_AW)][q] += ya * pw;
-    B.t[co_slot(e, CK_AE)][q] += ya * pe;
-    B.t[co_slot(e, CK_AS)][q] += ya * ps;
-    B.t[co_slot(e, CK_AN)][q] += ya * pn;
-    B.t[co_slot(e, CK_AP)][q] += -(ya * val);
-    B.t[co_slot(e, CK_SU)][q] += ya;
-    double *b = B.t[phi];
-    atomicAdd(b + q - 1, ya * aw);
-    atomicAdd(b + q + 1, ya * ae);
-    atomicAdd(b + q - nx, ya * as);
-    atomicAdd(b + q + nx, ya * an);
+    b[0] = 0.0;
+    const double ya = yb / k[CK_AP];
+    B.t[co_slot(e, CK_AW)][q] = bk[CK_AW] + ya * pw;
+    B.t[co_slot(e, CK_AE)][q] = bk[CK_AE] + ya * pe;
+    B.t[co_slot(e, CK_AS)][q] = bk[CK_AS] + ya * ps;
+    B.t[co_slot(e, CK_AN)][q] = bk[CK_AN] + ya * pn;
+    B.t[co_slot(e, CK_AP)][q] = bk[CK_AP] + -(ya * val);
+    B.t[co_slot(e, CK_SU)][q] = bk[CK_SU] + ya;
+    atomicAdd(b - 1, ya * k[CK_AW]);
+    atomicAdd(b + 1, ya * k[CK_AE]);
+    atomicAdd(b - nx, ya * k[CK_AS]);
+    atomicAdd(b + nx, ya * k[CK_AN]);
 }
 
 // ------------------------------- closed-form transposes: the assembly family
@@ -897,25 +971,80 @@ __device__ void prol_apply_adj(const LevelDev &F, const LevelDev &K, const Bars 
     }
 }
 
-// The closed-form transpose of one cell of phase P, for the kinds that have one;
-// false: transpose it by probes.
-__device__ __forceinline__ bool adj_closed(const CaseDev &C, const CaseTan &B, const Phase &P, int i, int j,
-                                           ParAcc &pa)
+// The copies: outflow's ghosts, the obstacle pressure copy, Jacobi's ring and copy back.
+__device__ __forceinline__ void pass_on(const Bars &b, int to, int qt, int from, int qf)
+{
+    b.add(from, qf, b.take(to, qt));
+}
+
+// P_JAC_SWEEP at cell q: new = (sum a_nb phi_nb + su) / (ap + 1e-30) from the old values
+// `cur` into `nxt` (adj_gs_cell's partials; the weight of the old value is 0).  `val`: the
+// new value.
+__device__ void jacobi_adj(const LevelDev &L, const Bars &b, int e, int cur, int nxt, int q, double val)
+{
+    const double y = b.take(nxt, q);
+    if (y == 0.0) return;
+    const int nx = L.npx;
+    const double *f = L.f[cur];
+    const double ya = y / (L.f[co_slot(e, CK_AP)][q] + 1.0e-30);
+    auto own = [&](int k, double v) { b.B.t[co_slot(e, k)][q] += v; };   // read by this cell alone
+    own(CK_AW, ya * f[q - 1]);
+    own(CK_AE, ya * f[q + 1]);
+    own(CK_AS, ya * f[q - nx]);
+    own(CK_AN, ya * f[q + nx]);
+    own(CK_AP, -(ya * val));
+    own(CK_SU, ya);
+    b.add(cur, q - 1, ya * L.f[co_slot(e, CK_AW)][q]);
+    b.add(cur, q + 1, ya * L.f[co_slot(e, CK_AE)][q]);
+    b.add(cur, q - nx, ya * L.f[co_slot(e, CK_AS)][q]);
+    b.add(cur, q + nx, ya * L.f[co_slot(e, CK_AN)][q]);
+}
+
+// Restore what phase P overwrote at cell (i, j) and transpose the cell in closed form.
+__device__ __forceinline__ void adj_closed(const CaseDev &C, const CaseTan &B, const CaseAdj &A, const Phase &P, int i,
+                                           int j, ParAcc &pa)
 {
     const LevelDev &F = C.lv[P.ig];
     const Bars bf{B.lv[P.ig]};
+    const int q = j * F.npx + i;
+    double val = 0.0;
+    if (P.kind == P_JAC_SWEEP) val = F.f[P.b == 0 ? tmp_of(P.a) : field_of(P.a)][q];
+    tape_cell(C, A, P, i, j, false);
     switch (P.kind) {
-    case P_ASM_U: asm_u_adj(C, F, bf, i, j, pa); return true;
-    case P_ASM_V: asm_v_adj(C, F, bf, i, j, pa); return true;
-    case P_ASM_SC: asm_sc_adj(F, bf, i, j, pa); return true;
-    case P_FINE_RES: fine_res_adj(F, bf, i, j, P.a, pa); return true;
-    case P_RESTRICT: restrict_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a, pa); return true;
-    case P_MASS_COEFP: mass_coefp_adj(C, F, bf, i, j, P.a); return true;
-    case P_RESTV: restv_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); return true;
-    case P_PROL_CORR: prol_corr_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); return true;
-    case P_PROL_APPLY: prol_apply_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); return true;
-    case P_UPDATE: update_adj(C, F, bf, j * F.npx + i, P.a); return true;
-    default: return false;
+    case P_ASM_U: asm_u_adj(C, F, bf, i, j, pa); break;
+    case P_ASM_V: asm_v_adj(C, F, bf, i, j, pa); break;
+    case P_ASM_SC: asm_sc_adj(F, bf, i, j, pa); break;
+    case P_SC_OUTFLOW: pass_on(bf, S_SC, q, S_SC, q - 1); break;
+    case P_JAC_RING: pass_on(bf, tmp_of(P.a), q, field_of(P.a), q); break;
+    case P_JAC_COPY: pass_on(bf, field_of(P.a), q, tmp_of(P.a), q); break;
+    case P_JAC_SWEEP:
+        if (P.b == 0) jacobi_adj(F, bf, P.a, field_of(P.a), tmp_of(P.a), q, val);
+        else jacobi_adj(F, bf, P.a, tmp_of(P.a), field_of(P.a), q, val);
+        break;
+    case P_PFIX: pass_on(bf, S_P, F.pdst[i], S_P, F.psrc[i]); break;
+    case P_PFIX_GATHER: {
+        const double y = bf.B.pbuf_t[i];
+        bf.B.pbuf_t[i] = 0.0;
+        bf.add(S_P, F.psrc[i], y);
+        break;
+    }
+    case P_PFIX_SCATTER: bf.B.pbuf_t[i] += bf.take(S_P, F.pdst[i]); break;
+    case P_OUTFLOW: {
+        const int g = j * F.npx + F.npx - 1;
+        pass_on(bf, S_U, g - 1, S_U, g - 2);
+        pass_on(bf, S_V, g, S_V, g - 1);
+        pass_on(bf, S_P, g, S_P, g - 1);
+        if (P.b) pass_on(bf, S_SC, g, S_SC, g - 1);
+        break;
+    }
+    case P_FINE_RES: fine_res_adj(F, bf, i, j, P.a, pa); break;
+    case P_RESTRICT: restrict_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a, pa); break;
+    case P_MASS_COEFP: mass_coefp_adj(C, F, bf, i, j, P.a); break;
+    case P_RESTV: restv_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); break;
+    case P_PROL_CORR: prol_corr_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); break;
+    case P_PROL_APPLY: prol_apply_adj(F, C.lv[P.ig + 1], bf, Bars{B.lv[P.ig + 1]}, i, j, P.a); break;
+    case P_UPDATE: update_adj(C, F, bf, q, P.a); break;
+    default: break;
     }
 }
 
@@ -937,61 +1066,93 @@ __device__ __forceinline__ void flush_par(ParAcc &pa, const Phase &P, double *pa
     pa = ParAcc{0.0, 0.0, 0.0, 0.0};
 }
 
+__device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes)
+{
+    for (int k = threadIdx.x; k < bytes / 8; k += blockDim.x)
+        static_cast<unsigned long long *>(dst)[k] = static_cast<const unsigned long long *>(src)[k];
+}
+static_assert(sizeof(CaseDev) % 8 == 0 && sizeof(CaseTan) % 8 == 0 && sizeof(Phase) % 8 == 0, "copied by words");
+
 // One V-cycle of case blockIdx.y, taped, then its transpose, on a cluster of
 // gridDim.x CTAs (the cluster is the case: every phase is spread over its threads and
 // separated from the next by a cluster barrier).  No thread leaves before the last
 // barrier: every CTA of the cluster takes the same phases.
-__global__ void __launch_bounds__(ADJ_BLOCK, 1) k_adj_cycle(const CaseDev *__restrict__ cs, CaseState *st,
-                                                            const CaseTan *__restrict__ ts, const CaseAdj *__restrict__ as)
+// (left to itself the compiler outlines the cells' bodies once there are several
+// instantiations, at 10% of the cycle)
+#define INLINE_CELL __attribute__((always_inline))
+template <bool GENERIC, int NT>
+__global__ void __launch_bounds__(NT, 1) k_adj_cycle(const CaseDev *__restrict__ cs, CaseState *st,
+                                                            const CaseTan *__restrict__ ts, const CaseAdj *__restrict__ as,
+                                                            int prog_cap)
 {
+    // The case's tables and program in shared memory: a barrier's acquire drops what L1
+    // holds, so from global memory every pass would fetch its phase, then its level's
+    // pointers, then its data, one L2 round trip after the other.
     __shared__ int bad_s;
-    const CaseDev &C = cs[blockIdx.y];
-    const CaseAdj &A = as[blockIdx.y];
-    const CaseTan &B = ts[blockIdx.y];
+    __shared__ CaseDev C;
+    __shared__ CaseTan B;
+    extern __shared__ Phase prog_s[];
+    CaseAdj A = as[blockIdx.y];
     if (A.nphase <= 0) return;   // the same for every CTA of the cluster
+    copy_words(&C, cs + blockIdx.y, sizeof(CaseDev));
+    copy_words(&B, ts + blockIdx.y, sizeof(CaseTan));
+    if (A.nphase <= prog_cap) {
+        copy_words(prog_s, A.prog, A.nphase * (int)sizeof(Phase));
+        A.prog = prog_s;
+    }
     if (threadIdx.x == 0) bad_s = 0;
     __syncthreads();
     int bad = 0;
-    // forward, taped (a half-sweep tapes and updates each cell in one pass)
+    // forward, taped: each cell saves and runs in one pass, a group of independent phases
+    // between two barriers.  Bound by the passes' latency (a barrier and an L2 round trip
+    // each): phase by phase, with a barrier between the saving and the run, a cycle of six
+    // 128^2 cases took 864 passes and 5.5 ms; by groups it takes 372, 2.8 ms.  The probes'
+    // check (GENERIC) keeps the phases apart.
+    int base = 0;
     for (int p = 0; p < A.nphase; ++p) {
         const Phase P = A.prog[p];
-        if (P.kind == P_GS && !A.generic) {
-            double *tape = A.tape + P.off;
-            gs_cells(C.lv[P.ig], P, [&](int i, int j, int t) { fwd_gs_cell(C.lv[P.ig], P.a, i, j, tape, t); });
+        if (GENERIC) {
+            tape_copy(C, A, P, true);
             case_barrier();
-            continue;
         }
-        tape_copy(C, A, P, true);
-        case_barrier();
-        const RecCase X{C, write_level(P), write_mask(P), &bad};
-        phase_cells(C, P, [&](int i, int j) { phase_cell(X, P, i, j); });
-        case_barrier();
+        if (P.kind == P_GS && !GENERIC) {
+            double *tape = A.tape + P.off;
+            gs_cells(C.lv[P.ig], P, base, [&](int i, int j, int t) INLINE_CELL { fwd_gs_cell(C.lv[P.ig], P.a, i, j, tape, t); });
+        } else {
+            const RecCase X{C, write_level(P), write_mask(P), &bad};
+            phase_cells(C, P, base, [&](int i, int j) INLINE_CELL {
+                if (!GENERIC) tape_cell(C, A, P, i, j, true);
+                phase_cell(X, P, i, j);
+            });
+        }
+        if (P.sync || GENERIC) {
+            case_barrier();
+            base = 0;
+        }
     }
-    // reverse
+    // reverse: a group ends before the phase that ends the group before it
     ParAcc pa{0.0, 0.0, 0.0, 0.0};
     for (int p = A.nphase - 1; p >= 0; --p) {
         const Phase P = A.prog[p];
-        if (P.kind == P_GS && !A.generic) {
-            const double *tape = A.tape + P.off;
-            gs_cells(C.lv[P.ig], P,
-                     [&](int i, int j, int t) { adj_gs_cell(C.lv[P.ig], B.lv[P.ig], P.a, i, j, tape, t); });
+        if (GENERIC) {
+            tape_copy(C, A, P, false);
             case_barrier();
-            continue;
+            phase_cells(C, P, base, [&](int i, int j) INLINE_CELL { adj_cell(C, B, P, i, j, pa, &bad); });
+        } else if (P.kind == P_GS) {
+            const double *tape = A.tape + P.off;
+            gs_cells(C.lv[P.ig], P, base,
+                     [&](int i, int j, int t) INLINE_CELL { adj_gs_cell(C.lv[P.ig], B.lv[P.ig], P.a, i, j, tape, t); });
+        } else {
+            phase_cells(C, P, base, [&](int i, int j) INLINE_CELL { adj_closed(C, B, A, P, i, j, pa); });
         }
-        tape_copy(C, A, P, false);
-        case_barrier();
-        {
-            const bool closed = !A.generic && (P.kind == P_ASM_U || P.kind == P_ASM_V || P.kind == P_ASM_SC ||
-                                               P.kind == P_FINE_RES || P.kind == P_RESTRICT ||
-                                               P.kind == P_MASS_COEFP || P.kind == P_UPDATE || P.kind == P_RESTV ||
-                                               P.kind == P_PROL_CORR || P.kind == P_PROL_APPLY);
-            if (closed)
-                phase_cells(C, P, [&](int i, int j) { adj_closed(C, B, P, i, j, pa); });
-            else
-                phase_cells(C, P, [&](int i, int j) { adj_cell(C, B, P, i, j, pa, &bad); });
+        // the kinds that read amu or amusc
+        if (P.kind == P_ASM_U || P.kind == P_ASM_V || P.kind == P_ASM_SC || P.kind == P_FINE_RES ||
+            P.kind == P_RESTRICT)
             flush_par(pa, P, A.pacc);
+        if (GENERIC || p == 0 || A.prog[p - 1].sync) {
+            case_barrier();
+            base = 0;
         }
-        case_barrier();
     }
     if (bad) atomicOr(&bad_s, 1);
     __syncthreads();
@@ -1026,7 +1187,7 @@ bool build_adj_program(const CaseDev &hc, const Sched &S, std::vector<Phase> &pr
     if (hc.ibc_xm == 3 || hc.ibc_xp == 3 || hc.ibc_ym == 3 || hc.ibc_yp == 3) return false;
     const int ng = hc.ngrid;
     auto add = [&](int kind, int ig, int a = 0, int b = 0) {
-        Phase P{kind, ig, a, b, tape};
+        Phase P{kind, ig, a, b, tape, 0};
         const LevelDev &L = hc.lv[write_level(P)];
         const unsigned long long m = write_mask(P);
         long long n = 0;
@@ -1041,17 +1202,26 @@ bool build_adj_program(const CaseDev &hc, const Sched &S, std::vector<Phase> &pr
         tape += n;
         prog.push_back(P);
     };
+    auto end_group = [&]() {
+        if (!prog.empty()) prog.back().sync = 1;
+    };
     auto smooth = [&](int ig, const int *eqs, int ne, int nsw) {
         if (nsw <= 0) return;
         if (S.isolve == MGFVM_JACOBI) {
             for (int k = 0; k < ne; ++k) add(P_JAC_RING, ig, eqs[k]);
-            for (int it = 0; it < nsw; ++it)
+            end_group();
+            for (int it = 0; it < nsw; ++it) {
                 for (int k = 0; k < ne; ++k) add(P_JAC_SWEEP, ig, eqs[k], it & 1);
+                end_group();
+            }
             if (nsw & 1)
                 for (int k = 0; k < ne; ++k) add(P_JAC_COPY, ig, eqs[k]);
+            end_group();
         } else if (S.isolve == MGFVM_GAUSS_SEIDEL) {
-            for (int h = 0; h < 2 * nsw; ++h)
+            for (int h = 0; h < 2 * nsw; ++h) {
                 for (int k = 0; k < ne; ++k) add(P_GS, ig, eqs[k], h & 1);
+                end_group();
+            }
         }
     };
     // one SIMPLE step on level ig (down leg :201-207, up leg :235-244)
@@ -1061,41 +1231,51 @@ bool build_adj_program(const CaseDev &hc, const Sched &S, std::vector<Phase> &pr
         add(P_ASM_V, ig);
         add(P_ASM_SC, ig);
         if (down && hc.ibc_xp == 4) add(P_SC_OUTFLOW, ig);
+        end_group();   // the assemblies read none of the scalar
         smooth(ig, uvsc, 3, S.nswpm);
         // multi-output routines run one output group per phase: a transposed phase then
         // probes only the reads of that group
         add(P_MASS_COEFP, ig, MC_COEF);
         add(P_MASS_COEFP, ig, MC_SU);
+        end_group();
         smooth(ig, pp, 1, S.nswpp);
         for (int part = 1; part <= 4; part <<= 1) add(P_UPDATE, ig, part);
+        end_group();
         if (hc.lv[ig].ncopy > 0) {
             if (hc.lv[ig].hazard) {
                 add(P_PFIX_GATHER, ig);
+                end_group();
                 add(P_PFIX_SCATTER, ig);
             } else {
                 add(P_PFIX, ig);
             }
+            end_group();
         }
         if (hc.ibc_xp == 4) add(P_OUTFLOW, ig, 0, down ? 0 : 1);
+        end_group();
     };
     for (int ig = 0; ig < ng; ++ig) {
         step(ig, true);
         if (ig != ng - 1) {
             for (int part = 1; part <= 8; part <<= 1) add(P_RESTV, ig, part);
             for (int w = 0; w < 3; ++w) add(P_FINE_RES, ig, w);
+            end_group();   // restv writes the coarse state, the residuals the fine buffers
             for (int w = 0; w < 3; ++w) add(P_RESTRICT, ig, w);
+            end_group();
         }
     }
     for (int ig = ng - 1; ig > 0; --ig) {
         for (int part = 1; part <= 8; part <<= 1) add(P_PROL_CORR, ig - 1, part);
+        end_group();
         for (int part = 1; part <= 8; part <<= 1) add(P_PROL_APPLY, ig - 1, part);
+        end_group();
         if (ig != 1) step(ig - 1, false);
     }
     return true;
 }
 
 cudaError_t launch_adj_cycle(const CaseDev *dc, CaseState *ds, const CaseTan *dt, const CaseAdj *da, int ncases,
-                             int cluster, cudaStream_t st)
+                             int cluster, bool small, bool generic, cudaStream_t st)
 {
     if (cluster < 1 || cluster > 8) return cudaErrorInvalidValue;
     cudaLaunchAttribute at[1];
@@ -1105,11 +1285,14 @@ cudaError_t launch_adj_cycle(const CaseDev *dc, CaseState *ds, const CaseTan *dt
     at[0].val.clusterDim.z = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)cluster, (unsigned)ncases, 1);
-    c.blockDim = dim3(ADJ_BLOCK, 1, 1);
+    c.blockDim = dim3((unsigned)(small && !generic ? ADJ_BLOCK_SMALL : ADJ_BLOCK), 1, 1);
+    c.dynamicSmemBytes = ADJ_PROG_MAX * sizeof(Phase);
     c.stream = st;
     c.attrs = at;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k_adj_cycle, dc, ds, dt, da);
+    if (generic) return cudaLaunchKernelEx(&c, k_adj_cycle<true, ADJ_BLOCK>, dc, ds, dt, da, (int)ADJ_PROG_MAX);
+    if (small) return cudaLaunchKernelEx(&c, k_adj_cycle<false, ADJ_BLOCK_SMALL>, dc, ds, dt, da, (int)ADJ_PROG_MAX);
+    return cudaLaunchKernelEx(&c, k_adj_cycle<false, ADJ_BLOCK>, dc, ds, dt, da, (int)ADJ_PROG_MAX);
 }
 
 int adj_cluster_size(int ncases, int sms)

@@ -9,8 +9,8 @@
 // sweep run each phase as one parallel pass and lets its transpose be formed cell by
 // cell:
 //
-//   forward (taped)  before each phase, copy the arrays it overwrites to a tape; run it.
-//   reverse          for each phase, last to first: restore its overwritten arrays from
+//   forward (taped)  before each phase, copy what it overwrites to a tape; run it.
+//   reverse          for each phase, last to first: restore what it overwrote from
 //                    the tape (the state is then its input), then for every cell
 //                      1. evaluate the cell routine once, reading the adjoints of the
 //                         values it writes and clearing them (the writes replace them),
@@ -53,9 +53,12 @@ enum PhaseKind {
 
 // One phase of a case's V-cycle program; `off` is the tape offset (doubles) of the
 // arrays it overwrites.
+// `sync`: the next phase needs this one finished; the phases up to such a one are
+// independent of each other (none reads or writes what another writes) and run together.
 struct Phase {
     int kind, ig, a, b;
     long long off;
+    long long sync;
 };
 
 // What a case's adjoint kernel reads: its program, tape, and the per-level adjoints
@@ -65,7 +68,6 @@ struct CaseAdj {
     int nphase;
     double *tape;
     double *pacc;
-    int generic;   // transpose every phase by dual-number probes (the closed forms' check)
 };
 
 // Bit `s` of the mask: slot s of the written level; PB_BIT: the pressure-copy buffer.
@@ -79,9 +81,11 @@ bool build_adj_program(const CaseDev &hc, const Sched &S, std::vector<Phase> &pr
 // One V-cycle of every case, taped, then its transpose: the adjoint arrays `dt` (the
 // derivative storage of mg_tangent.cuh, one array per differentiable slot) go from the
 // adjoint of the state after the cycle to that of the state before it.  A cluster of
-// `cluster` (1..8) CTAs per case; a case with an empty program is skipped.
+// `cluster` (1..8) CTAs per case, of ADJ_BLOCK_SMALL threads with `small`; a case with an
+// empty program is skipped.  `generic`:
+// transpose every phase by dual-number probes (the closed forms' check).
 cudaError_t launch_adj_cycle(const CaseDev *dc, CaseState *ds, const CaseTan *dt, const CaseAdj *da, int ncases,
-                             int cluster, cudaStream_t st);
+                             int cluster, bool small, bool generic, cudaStream_t st);
 
 // CTAs per case of launch_adj_cycle for a batch of `ncases` on `sms` multiprocessors:
 // the largest power of two up to 8 that keeps every case's cluster resident at once.
@@ -92,6 +96,11 @@ int adj_cluster_size(int ncases, int sms);
 cudaError_t launch_live_copy(const CaseDev *dc, const long long *off, double *buf, int ncases, int maxcells,
                              int maxng, int dir, cudaStream_t st);
 
-constexpr int ADJ_BLOCK = 1024;
+// Threads of a CTA: 512 (128 registers each) where the finest level has at most
+// ADJ_SMALL_CELLS cells, whose passes are bound by latency, else 1024 (64).  Six 128^2 cases
+// 2.76 against 2.99 ms a cycle, sixteen 256^2 cases 17.9 against 16.2.
+constexpr int ADJ_BLOCK = 1024, ADJ_BLOCK_SMALL = 512;
+constexpr int ADJ_SMALL_CELLS = 20000;
+constexpr int ADJ_PROG_MAX = 700;   // phases kept in shared memory (longer programs are read from global)
 
 }  // namespace mg

@@ -2220,10 +2220,9 @@ int mgfvm_adjoint(mgfvm_ctx *x, int ncycles)
         for (auto &pg : progs) flat.insert(flat.end(), pg.begin(), pg.end());
         std::vector<CaseAdj> ha(n);
         const char *gen = std::getenv("MGFVM_ADJOINT_GENERIC");
-        const int generic = gen && std::atoi(gen) == 1 ? 1 : 0;
+        const bool generic = gen && std::atoi(gen) == 1;
         for (int c = 0; c < n; ++c)
-            ha[c] = CaseAdj{dprog + prog_off[c], (int)progs[c].size(), tape + tape_off[c], pacc + (size_t)c * 2 * MAXLEV,
-                            generic};
+            ha[c] = CaseAdj{dprog + prog_off[c], (int)progs[c].size(), tape + tape_off[c], pacc + (size_t)c * 2 * MAXLEV};
         if (cudaMemcpy(dprog, flat.data(), sizeof(Phase) * flat.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(dadj, ha.data(), sizeof(CaseAdj) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(dlive, live_off.data(), sizeof(long long) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2288,7 +2287,7 @@ int mgfvm_adjoint(mgfvm_ctx *x, int ncycles)
             for (int k = cnt - 1; k >= 0 && rc == MGFVM_OK; --k) {
                 rc = live(seg + (size_t)k * live_tot, 1);
                 if (rc != MGFVM_OK) break;
-                cudaError_t e = launch_adj_cycle(x->dc, x->ds, x->dt, dadj, n, cluster, x->stream);
+                cudaError_t e = launch_adj_cycle(x->dc, x->ds, x->dt, dadj, n, cluster, maxcells <= ADJ_SMALL_CELLS, generic, x->stream);
                 if (e != cudaSuccess) rc = mgfvm_fail(MGFVM_ECUDA, "adjoint cycle: %s", cudaGetErrorString(e));
                 x->launches += 1;
             }
