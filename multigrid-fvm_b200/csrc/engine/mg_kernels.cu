@@ -23,6 +23,7 @@
 #include "mg_reduce.cuh"
 #include "mg_tangent.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace mg {
@@ -406,10 +407,11 @@ struct PairTile {
 };
 
 // 0: this CTA has work, 1: it has none, 2: the launch is too small for its region.
-// `bx` picks the tile (blockIdx.x in the tiled smoothers).
-__device__ __forceinline__ int pair_tile(const LevelDev &L, int e, int nu, int tile, PairTile &P, int bx)
+// `bx` picks the tile (blockIdx.x in the tiled smoothers) of the domain, whose rows are npx
+// cells apart.
+__device__ __forceinline__ int pair_tile(const Dom &dom, int npx, int nu, int tile, PairTile &P, int bx)
 {
-    P.d = dom_eq(L, e);
+    P.d = dom;
     const Dom &d = P.d;
     if (d.wi <= 0 || d.wj <= 0) return 1;
     const int tx_n = (d.wi + tile - 1) / tile, ty_n = (d.wj + tile - 1) / tile;
@@ -440,8 +442,8 @@ __device__ __forceinline__ int pair_tile(const LevelDev &L, int e, int nu, int t
     P.okB = own && (P.jB == jr || two);
     P.kA = (P.jA - P.ry0) * W + c;
     P.kB = (P.jB - P.ry0) * W + c;
-    P.gA = P.jA * L.npx + i;
-    P.gB = P.jB * L.npx + i;
+    P.gA = P.jA * npx + i;
+    P.gB = P.jB * npx + i;
     const bool inx = i >= d.i0 && i <= P.dx1;
     const int dxe = min(i - P.x0, P.x1 - i);
     P.limA = P.okA && inx && P.jA >= d.j0 && P.jA <= P.dy1 ? H + min(dxe, min(P.jA - P.y0, P.y1 - P.jA)) : -1;
@@ -451,6 +453,10 @@ __device__ __forceinline__ int pair_tile(const LevelDev &L, int e, int nu, int t
     P.outA = P.okA && outx && P.jA >= oy0 && P.jA <= oy1;
     P.outB = P.okB && outx && P.jB >= oy0 && P.jB <= oy1;
     return 0;
+}
+__device__ __forceinline__ int pair_tile(const LevelDev &L, int e, int nu, int tile, PairTile &P, int bx)
+{
+    return pair_tile(dom_eq(L, e), L.npx, nu, tile, P, bx);
 }
 
 // Temporal-blocked smoother.  blockIdx.z picks an equation of `mask`, blockIdx.x a
@@ -1919,6 +1925,59 @@ __global__ void __launch_bounds__(BLOCK) r_jacobi(const double *__restrict__ aw,
                           cur[q + npx], cur[q]);
 }
 
+// Jacobi by tiles: `nu` sweeps of the tile plus a halo of one cell a sweep in shared memory
+// (k_smooth on a caller's level), from src to dst.
+__global__ void __launch_bounds__(SMOOTH_BLOCK, 1)
+    r_jacobi_tile(const double *__restrict__ aw, const double *__restrict__ ae, const double *__restrict__ as,
+                  const double *__restrict__ an, const double *__restrict__ ap, const double *__restrict__ su,
+                  const double *src, double *dst, int npx, int wi, int wj, int nu, int tile)
+{
+    extern __shared__ double sm[];
+    PairTile P;
+    if (pair_tile(Dom{1, 1, wi, wj}, npx, nu, tile, P, blockIdx.x) != 0) {
+        pdl_enter();
+        return;   // (the launch is sized to its tiles)
+    }
+    const int W = P.W, k2[2] = {P.kA, P.kB}, g2[2] = {P.gA, P.gB}, lim[2] = {P.limA, P.limB};
+    const bool ok[2] = {P.okA, P.okB}, out[2] = {P.outA, P.outB};
+    double *phi = sm, *phi2 = sm + W * P.Hh;
+    double c[2][6], v[2] = {0.0, 0.0};
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        c[x][0] = c[x][1] = c[x][2] = c[x][3] = 0.0;
+        c[x][4] = c[x][5] = 1.0;
+        if (lim[x] >= 0) {
+            const int g = g2[x];
+            c[x][0] = aw[g]; c[x][1] = ae[g]; c[x][2] = as[g]; c[x][3] = an[g]; c[x][4] = ap[g]; c[x][5] = su[g];
+        }
+    }
+    pdl_enter();
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (ok[x]) v[x] = src[g2[x]];
+    const Recip R[2] = {make_recip(c[0][4] + 1.0e-30), make_recip(c[1][4] + 1.0e-30)};
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (ok[x]) phi[k2[x]] = phi2[k2[x]] = v[x];
+    __syncthreads();
+    for (int h = 1; h <= nu; ++h) {
+        const double *cur = ((h - 1) & 1) ? phi2 : phi;
+        double *nxt = ((h - 1) & 1) ? phi : phi2;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (h <= lim[x]) {
+                const int k = k2[x];
+                v[x] = jacobi_value_r(c[x][0], c[x][1], c[x][2], c[x][3], R[x], c[x][5], cur[k - 1], cur[k + 1],
+                                      cur[k - W], cur[k + W], cur[k]);
+                nxt[k] = v[x];
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (out[x]) dst[g2[x]] = v[x];
+}
+
 __global__ void __launch_bounds__(BLOCK) r_copy(const double *src, double *dst, int npx, int nx, int ny)
 {
     const int wi = nx - 1, t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1942,26 +2001,39 @@ __global__ void __launch_bounds__(BLOCK) r_gs(const double *__restrict__ aw, con
     phi[q] = gs_value(aw[q], ae[q], as[q], an[q], ap[q], su[q], phi[q - 1], phi[q + 1], phi[q - npx], phi[q + npx]);
 }
 
+// Bound by memory (48 bytes a cell) once the level outgrows the end of the reduction: PER
+// cells a thread, whose loads are in flight together, mean as many fewer partial sums to
+// publish and to gather.  `slots`: the partials' length, after which the counter lies.
+template <int PER>
 __global__ void __launch_bounds__(BLOCK) r_masserror(const double *u, const double *v, const double *ax,
                                                      const double *ay, double *su, double *pp, int npx,
-                                                     int npy, double *err_out, double *partials)
+                                                     int npy, double *err_out, double *partials, int slots)
 {
-    const int wi = npx - 2, n = wi * (npy - 2), nb = (n + blockDim.x - 1) / blockDim.x;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double a[1] = {0.0};
-    if (t < n) {
-        const int q = (1 + t / wi) * npx + 1 + t % wi;
-        const double axq = ax[q], ayq = ay[q];
-        double div = axq * u[q] - axq * u[q - 1] + ayq * v[q] - ayq * v[q - npx];
-        su[q] = -div;
-        pp[q] = 0.0;
-        a[0] = fabs(div);
+    const int wi = npx - 2, n = wi * (npy - 2);
+    int q[PER];
+    double x[PER][6], a[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int t = (blockIdx.x * PER + k) * BLOCK + threadIdx.x;
+        q[k] = t < n ? (1 + t / wi) * npx + 1 + t % wi : 0;
+        if (q[k]) {
+            x[k][0] = ax[q[k]]; x[k][1] = ay[q[k]];
+            x[k][2] = u[q[k]]; x[k][3] = u[q[k] - 1]; x[k][4] = v[q[k]]; x[k][5] = v[q[k] - npx];
+        }
     }
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+        if (q[k]) {
+            const double div = x[k][0] * x[k][2] - x[k][0] * x[k][3] + x[k][1] * x[k][4] - x[k][1] * x[k][5];
+            su[q[k]] = -div;
+            pp[q[k]] = 0.0;
+            a[0] += fabs(div);
+        }
     block_sum<1>(a);
-    unsigned *counter = reinterpret_cast<unsigned *>(partials + (size_t)nb * RED_STRIDE);
-    if (publish_partials<1>(partials, counter, a, nb)) {
+    unsigned *counter = reinterpret_cast<unsigned *>(partials + (size_t)slots * RED_STRIDE);
+    if (publish_partials<1>(partials, counter, a, gridDim.x)) {
         double s[1];
-        gather_partials<1>(partials, nb, s);
+        gather_partials<1>(partials, gridDim.x, s);
         if (threadIdx.x == 0) { *err_out = s[0]; *counter = 0; }
     }
 }
@@ -1974,6 +2046,51 @@ cudaError_t raw_jacobi(const double *aw, const double *ae, const double *as, con
 {
     (void)npy;
     if (nsw <= 0 || nx < 2 || ny < 2) return cudaSuccess;
+    // An even number of tile launches through the scratch (one in place where a tile holds
+    // the level) where they are expected to take less than a launch a sweep: a round of tile
+    // CTAs takes 5 us and 0.5 a sweep, a sweep over the level 4.1 us, 8.3 us a million cells
+    // where that is more (12 sweeps of 90 x 70: 45 us against 12 by tiles; four of
+    // 1024 x 1024: 37 against 51).
+    {
+        const int wi = nx - 1, wj = ny - 1;
+        const double plain = (nsw + (nsw & 1)) * std::max(4.1, 8.3e-6 * wi * wj);
+        int chunks = 0, tile = 0;
+        double best = plain;
+        if ((long long)(wi + 2) * ((wj + 3) / 2) <= SMOOTH_BLOCK) {
+            if (5.0 + 0.5 * nsw < best) {
+                chunks = 1;
+                tile = std::max(wi, wj);
+            }
+        } else {
+            for (int c = 2; c <= nsw; c += 2) {
+                const int u = (nsw + c - 1) / c, side = smooth_pairs_side(u, SMOOTH_BLOCK);
+                if (side < MIN_TILE) continue;
+                const long long n = (long long)((wi + side - 1) / side) * ((wj + side - 1) / side);
+                const double t = c * (double)((n + 147) / 148) * (5.0 + 0.5 * u);
+                if (t < best) {
+                    best = t;
+                    chunks = c;
+                    tile = side;
+                }
+            }
+        }
+        if (chunks > 0) {
+            const int hmax = (nsw + chunks - 1) / chunks;
+            const int side = chunks == 1 ? 0 : tile + 2 * hmax, cells = chunks == 1 ? (wi + 2) * (wj + 2) : side * side;
+            const int pairs = chunks == 1 ? (wi + 2) * ((wj + 3) / 2) : side * ((side + 1) / 2);
+            const int block = std::min(SMOOTH_BLOCK, (pairs + 31) / 32 * 32);
+            const dim3 grid(((wi + tile - 1) / tile) * ((wj + tile - 1) / tile));
+            for (int c = 0; c < chunks; ++c) {
+                const int nu = nsw / chunks + (c < nsw % chunks ? 1 : 0);
+                const double *src = (c & 1) ? scratch : phi;
+                double *dst = (c & 1) || chunks == 1 ? phi : scratch;
+                const cudaError_t e = launch_k(c > 0, r_jacobi_tile, grid, block, 2 * cells * (int)sizeof(double), s, aw,
+                                               ae, as, an, ap, su, src, dst, npx, wi, wj, nu, tile);
+                if (e != cudaSuccess) return e;
+            }
+            return cudaSuccess;
+        }
+    }
     for (int it = 0; it < nsw; ++it) {
         const double *cur = (it & 1) ? scratch : phi;
         double *nxt = (it & 1) ? phi : scratch;
@@ -2009,7 +2126,12 @@ cudaError_t raw_masserror(const double *u, const double *v, const double *ax, co
 {
     const int nb = (int)raw_masserror_blocks(npx, npy);
     if (nb == 0) return cudaMemsetAsync(err_out, 0, sizeof(double), s);
-    r_masserror<<<nb, BLOCK, 0, s>>>(u, v, ax, ay, su, pp, npx, npy, err_out, partials);
+    // (from four blocks an SM on: 512 x 512 in 6.2 us against 8.2, 1024 x 1024 in 12.3
+    // against 20.5; 400 x 300 in 6.2 either way)
+    if (nb >= 4 * 148)
+        r_masserror<8><<<(nb + 7) / 8, BLOCK, 0, s>>>(u, v, ax, ay, su, pp, npx, npy, err_out, partials, nb);
+    else
+        r_masserror<1><<<nb, BLOCK, 0, s>>>(u, v, ax, ay, su, pp, npx, npy, err_out, partials, nb);
     return cudaGetLastError();
 }
 

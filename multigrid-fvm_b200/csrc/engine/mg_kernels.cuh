@@ -49,7 +49,7 @@ struct Launch {
     dim3 grid;
     int block;
     int smem;
-    int bw, bh;        // K_SMOOTH_TMA: box width and height
+    int bw, bh;        // K_SMOOTH_TMA: box width and height; K_SMOOTH_Q: tile
     int map;           // K_SMOOTH_TMA: index of its first tensor-map pair in the schedule's table
     const void *ptr;   // K_SMOOTH_TMA: that pair on the device (one per case)
 };
@@ -106,6 +106,12 @@ cudaError_t launch_tile(const Launch &L, const CaseDev *dcases, CaseState *dstat
 // every 2 x 4 cells, 12 warps: three on each partition of an SM, 168 registers a thread.
 constexpr int SMOOTH_Q_COLS = 54, SMOOTH_Q_ROWS = 56, SMOOTH_Q_THREADS = 384;
 cudaError_t launch_smooth_q(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
+
+// The same on a caller's own level (mgfvm_rbgs_f64): the expected time of its plan, and the
+// launches (`tmp` unused where chunks is 1).
+double raw_q_plan(int wi, int wj, int units, int &chunks, int &tw, int &th);
+cudaError_t raw_smooth_q(const double *const *co, double *phi, double *tmp, int npx, int wi, int wj, int units, int chunks,
+                         int tw, int th, cudaStream_t st);
 
 // Kernels of the raw-pointer entry points.
 cudaError_t raw_jacobi(const double *aw, const double *ae, const double *as, const double *an,

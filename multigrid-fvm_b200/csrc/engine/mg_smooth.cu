@@ -41,34 +41,32 @@ static_assert(QX * QY <= SMOOTH_Q_THREADS, "a thread a block");
 // shared-memory index of column 2 k + half of row r
 __device__ __forceinline__ int sh(int r, int half, int k) { return (r * 2 + half) * QX + k; }
 
-}  // namespace
+// One equation on one level: coefficients, where the field comes from and goes to (the same
+// array only where one tile covers the domain), row length and the domain [1, dx1] x [1, dy1].
+struct QIn {
+    const double *co[NCOEF], *src;
+    double *dst;
+    int npx, dx1, dy1;
+    bool vec;   // a block row's two cells may be loaded together (16-byte aligned)
+};
 
-// blockIdx.x: tile, .y: case, .z: equation of `mask`; `dir` 0: from the field to the
-// equation's ping-pong buffer, 1: the reverse.  tw x th: tile.  EARLY: a later launch of the
-// smoothing; its coefficients are read before waiting for the launch before it.
-template <bool EARLY>
-__global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
-    k_smooth_q(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int mask, int u0, int nu, int dir,
-               int tw, int th)
+// Tile (tx, ty) of tw x th cells.  `enter` waits for the launches before and says whether
+// the case is still running.  EARLY: the coefficients are read before that.
+template <bool EARLY, class Enter>
+__device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx, int ty, int tw, int th, int u0, int nu,
+                                              Enter enter)
 {
     __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
     double *phi = smq + 2 * QX;   // a row of slack on either side
-    const CaseDev &C = cs[blockIdx.y];
-    const FastLevel L = fast_level(C.lv[ig]);
-    const Fast io{L};
-    const int e = nth_eq(mask, blockIdx.z), npx = L.npx, t = threadIdx.x;
-    // the equation's domain [di, dx1] x [dj, dy1] = [1, ..]
-    const int dx1 = npx - (e == EQ_U ? 3 : 2), dy1 = L.npy - (e == EQ_V ? 3 : 2);
-    const int txn = max(1, (dx1 + tw - 1) / tw), tyn = (dy1 + th - 1) / th;
-    const bool active = mode_active(C, ig, mode) && dx1 >= 1 && dy1 >= 1 && (int)blockIdx.x < txn * tyn;
-    const int x0 = 1 + (blockIdx.x % txn) * tw, y0 = 1 + (blockIdx.x / txn) * th;
+    const int npx = in.npx, dx1 = in.dx1, dy1 = in.dy1, t = threadIdx.x;
+    const int x0 = 1 + tx * tw, y0 = 1 + ty * th;
     const int x1 = min(x0 + tw - 1, dx1), y1 = min(y0 + th - 1, dy1);
     const int cx0 = max(x0 - nu, 0) & ~1, cy0 = max(y0 - nu, 0) & ~1;
     const int rx1 = min(x1 + nu, dx1 + 1), ry1 = min(y1 + nu, dy1 + 1);
     const int qx = t % QX, qy = t / QX, i = cx0 + BX * qx, j = cy0 + BY * qy;
     const bool mine = active && qy < QY && i <= rx1 && j <= ry1;
     const int q0 = j * npx + i;
-    const bool vec = (npx & 1) == 0;
+    const bool vec = in.vec;
 
     // cell (x, y) of the block: k[y][x] = aw .. an, su, b, y; v = field
     double w[BY][BX], ea[BY][BX], so[BY][BX], no[BY][BX], su[BY][BX], b[BY][BX], rc[BY][BX], v[BY][BX];
@@ -95,18 +93,17 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
             }
     };
     auto coefs = [&]() {
-        load(io.at(co_slot(e, CK_AP)), b);
-        load(io.at(co_slot(e, CK_AW)), w);
-        load(io.at(co_slot(e, CK_AE)), ea);
-        load(io.at(co_slot(e, CK_AS)), so);
-        load(io.at(co_slot(e, CK_AN)), no);
-        load(io.at(co_slot(e, CK_SU)), su);
+        load(in.co[CK_AP], b);
+        load(in.co[CK_AW], w);
+        load(in.co[CK_AE], ea);
+        load(in.co[CK_AS], so);
+        load(in.co[CK_AN], no);
+        load(in.co[CK_SU], su);
     };
     if (EARLY) coefs();
-    pdl_enter();
+    const bool live = enter();
     if (!active) return;
-    const bool live = !st[blockIdx.y].done;
-    load(io.at(dir == 1 ? eq_tmp(e) : eq_field(e)), v);
+    load(in.src, v);
     if (!EARLY) coefs();
     if (!live) return;
     // cells outside the domain (the boundary ring, unused halo) are never updated; harmless
@@ -173,7 +170,6 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         __syncthreads();
     }
     // the tile, plus the boundary ring where it touches it
-    double *dst = io.at(dir == 0 ? eq_tmp(e) : eq_field(e));
     const int ox0 = x0 == 1 ? 0 : x0, ox1 = x1 == dx1 ? x1 + 1 : x1;
     const int oy0 = y0 == 1 ? 0 : y0, oy1 = y1 == dy1 ? y1 + 1 : y1;
     if (mine) {
@@ -181,8 +177,49 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         for (int y = 0; y < BY; ++y)
 #pragma unroll
             for (int x = 0; x < BX; ++x)
-                if (i + x >= ox0 && i + x <= ox1 && j + y >= oy0 && j + y <= oy1) dst[q0 + y * npx + x] = v[y][x];
+                if (i + x >= ox0 && i + x <= ox1 && j + y >= oy0 && j + y <= oy1) in.dst[q0 + y * npx + x] = v[y][x];
     }
+}
+
+}  // namespace
+
+// blockIdx.x: tile, .y: case, .z: equation of `mask`; `dir` 0: from the field to the
+// equation's ping-pong buffer, 1: the reverse.  EARLY: a later launch of the smoothing.
+template <bool EARLY>
+__global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
+    k_smooth_q(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int mask, int u0, int nu, int dir,
+               int tw, int th)
+{
+    const CaseDev &C = cs[blockIdx.y];
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
+    const int e = nth_eq(mask, blockIdx.z);
+    QIn in;
+    in.npx = L.npx;
+    in.dx1 = L.npx - (e == EQ_U ? 3 : 2);
+    in.dy1 = L.npy - (e == EQ_V ? 3 : 2);
+    in.vec = (L.npx & 1) == 0;
+#pragma unroll
+    for (int k = 0; k < NCOEF; ++k) in.co[k] = io.at(co_slot(e, k));
+    in.src = io.at(dir == 1 ? eq_tmp(e) : eq_field(e));
+    in.dst = io.at(dir == 0 ? eq_tmp(e) : eq_field(e));
+    const int txn = max(1, (in.dx1 + tw - 1) / tw), tyn = (in.dy1 + th - 1) / th;
+    const bool active = mode_active(C, ig, mode) && in.dx1 >= 1 && in.dy1 >= 1 && (int)blockIdx.x < txn * tyn;
+    smooth_q_tile<EARLY>(in, active, blockIdx.x % txn, blockIdx.x / txn, tw, th, u0, nu, [&]() {
+        pdl_enter();
+        return !active || !st[blockIdx.y].done;
+    });
+}
+
+// The same on a caller's own level.
+template <bool EARLY>
+__global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1) r_smooth_q(QIn in, int u0, int nu, int tw, int th)
+{
+    const int txn = (in.dx1 + tw - 1) / tw;
+    smooth_q_tile<EARLY>(in, true, blockIdx.x % txn, blockIdx.x / txn, tw, th, u0, nu, [&]() {
+        pdl_enter();
+        return true;
+    });
 }
 
 cudaError_t launch_smooth_q(const Launch &X, const CaseDev *dc, CaseState *ds, const Sched &S, cudaStream_t st)
@@ -192,6 +229,60 @@ cudaError_t launch_smooth_q(const Launch &X, const CaseDev *dc, CaseState *ds, c
                         X.a3 & 3, X.bw, X.bh);
     return launch_k(S.pdl, k_smooth_q<false>, X.grid, SMOOTH_Q_THREADS, 0, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2,
                     X.a3 & 3, X.bw, X.bh);
+}
+
+// The plan of `units` half-sweeps over a domain of wi x wj cells of one equation on a
+// caller's level, whose first and last launch read and write phi: one launch in place where
+// a region holds the whole level, else an even number through a buffer of the level's size.
+// Times in microseconds, as the schedule's for the engine's levels.
+double raw_q_plan(int wi, int wj, int units, int &chunks, int &tw, int &th)
+{
+    if (wi + 2 <= SMOOTH_Q_COLS && wj + 2 <= SMOOTH_Q_ROWS) {
+        chunks = 1;
+        tw = wi;
+        th = wj;
+        return 4.6 + 0.43 * units;
+    }
+    double best = 1e300;
+    auto side = [](int n, int most) { return (n + (n + most - 1) / most - 1) / ((n + most - 1) / most); };
+    for (int c = 2; c <= units; c += 2) {
+        const int u = (units + c - 1) / c, mx = SMOOTH_Q_COLS - 2 * u - 1, my = SMOOTH_Q_ROWS - 2 * u - 1;
+        if (mx < 8 || my < 8) continue;
+        const int w = side(wi, mx), h = side(wj, my);
+        const long long tiles = (long long)((wi + w - 1) / w) * ((wj + h - 1) / h);
+        const double t = c * (0.3 + (double)((tiles + 147) / 148) * (4.9 + 0.37 * u));
+        if (t < best) {
+            best = t;
+            chunks = c;
+            tw = w;
+            th = h;
+        }
+    }
+    return best;
+}
+
+cudaError_t raw_smooth_q(const double *const *co, double *phi, double *tmp, int npx, int wi, int wj, int units, int chunks,
+                         int tw, int th, cudaStream_t st)
+{
+    QIn in;
+    for (int k = 0; k < NCOEF; ++k) in.co[k] = co[k];
+    in.npx = npx;
+    in.dx1 = wi;
+    in.dy1 = wj;
+    in.vec = (npx & 1) == 0 && (((uintptr_t)phi | (uintptr_t)tmp) & 15) == 0;
+    for (int k = 0; k < NCOEF; ++k) in.vec = in.vec && ((uintptr_t)co[k] & 15) == 0;
+    const unsigned tiles = (unsigned)(((wi + tw - 1) / tw) * ((wj + th - 1) / th));
+    int u0 = 0;
+    for (int c = 0; c < chunks; ++c) {
+        const int nu = units / chunks + (c < units % chunks ? 1 : 0);
+        in.src = (c & 1) ? tmp : phi;
+        in.dst = (c & 1) || chunks == 1 ? phi : tmp;
+        const cudaError_t e = c == 0 ? launch_k(false, r_smooth_q<false>, dim3(tiles), SMOOTH_Q_THREADS, 0, st, in, u0, nu, tw, th)
+                                     : launch_k(true, r_smooth_q<true>, dim3(tiles), SMOOTH_Q_THREADS, 0, st, in, u0, nu, tw, th);
+        if (e != cudaSuccess) return e;
+        u0 += nu;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace mg
