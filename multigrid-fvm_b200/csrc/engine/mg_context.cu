@@ -58,6 +58,8 @@ struct mgfvm_ctx {
     std::vector<std::vector<int>> obs;
     std::vector<std::vector<double>> profile;
     std::vector<mgfvm_obstacle_prog> progs;   // ncases * MAXLEV
+    std::vector<int> prog_case;               // the case whose obstacle programs case c uses
+    const mgfvm_obstacle_prog &prog(int c, int ig) const { return progs[(size_t)prog_case[c] * MAXLEV + ig]; }
     std::vector<CaseDev> hc;
     std::vector<CaseState> hs;
     std::vector<InitDev> hinit;
@@ -69,6 +71,7 @@ struct mgfvm_ctx {
     double *hist = nullptr;
     int hist_cap = 0;
     double *dprofile = nullptr;
+    size_t profile_cap = 0;   // doubles dprofile holds
     int *dobs = nullptr;
     int *hflags = nullptr;                    // pinned readback of the per-case done flags, two sets
     size_t hflags_bytes = 0;
@@ -469,7 +472,7 @@ struct Builder {
         int maxcopy = 0, haz = 0;
         for (int c = 0; c < x->ncases; ++c) {
             if (!mode_active(x->hc[c], ig, mode)) continue;
-            const mgfvm_obstacle_prog &P = x->progs[c * MAXLEV + ig];
+            const mgfvm_obstacle_prog &P = x->prog(c, ig);
             maxcopy = std::max(maxcopy, P.ncopy);
             haz |= P.hazard;
         }
@@ -492,7 +495,7 @@ struct Builder {
             const CaseDev &C = x->hc[c];
             if (!mode_active(C, ig, mode)) continue;
             if (C.ibc_xm == 3 || C.ibc_ym == 3) return false;
-            if (!pfix_in_update && x->progs[(size_t)c * MAXLEV + ig].touches_outlet) return false;
+            if (!pfix_in_update && x->prog(c, ig).touches_outlet) return false;
         }
         return true;
     }
@@ -554,7 +557,7 @@ struct Builder {
     bool pfix_needed(int ig, int mode) const
     {
         for (int c = 0; c < x->ncases; ++c)
-            if (mode_active(x->hc[c], ig, mode) && x->progs[c * MAXLEV + ig].ncopy > 0) return true;
+            if (mode_active(x->hc[c], ig, mode) && x->prog(c, ig).ncopy > 0) return true;
         return false;
     }
     bool bound_needed(int bits) const
@@ -1019,7 +1022,7 @@ int alloc_tangent(mgfvm_ctx *x)
         for (int ig = 0; ig < g.ngrid; ++ig) {
             const size_t n = (size_t)npx_of(g, ig) * npy_of(g, ig);
             for (int s = 0; s < NSLOTS; ++s) offs[c].push_back(tangent_slot(s) ? take(n * sizeof(double)) : (size_t)-1);
-            const int nc = x->progs[(size_t)c * MAXLEV + ig].ncopy;
+            const int nc = x->prog(c, ig).ncopy;
             offs[c].push_back(take((size_t)std::max(nc, 1) * sizeof(double)));
         }
         x->tcase_bytes[c] = align_up(off, 256) - x->tcase_off[c];
@@ -1047,37 +1050,29 @@ int alloc_tangent(mgfvm_ctx *x)
     return MGFVM_OK;
 }
 
-// Zero case c's derivatives and seed its direction: the level-0 inlet face (i = 0,
-// row index + 1) with the coarse faces that rest_geom averages from it (rest_geom
-// :1391-1473, as k_rest_geom), or the derivative of every level's amu and amusc =
-// amuf / prsc (coefsc :867) with respect to amuf or prsc.
-int seed_tangent(mgfvm_ctx *x, int c)
+// Zero the derivatives of cases c0 .. c0 + n - 1 and seed their directions: the level-0
+// inlet face with the coarse faces that rest_geom averages from it (on the device), or the
+// derivative of every level's amu and amusc = amuf / prsc (coefsc :867) with respect to amuf
+// or prsc.
+int seed_tangent(mgfvm_ctx *x, int c0, int n)
 {
-    CK(cudaMemsetAsync(x->tpool + x->tcase_off[c], 0, x->tcase_bytes[c], x->stream));
-    const mgfvm_config &g = x->cfg[c];
-    const int kind = x->dir_kind[c], idx = x->dir_index[c];
-    for (int ig = 0; ig < g.ngrid; ++ig) {
-        LevelTan &D = x->ht[c].lv[ig];
-        D.amu_t = kind == MGFVM_DIR_AMUF ? 1.0 : 0.0;
-        D.amusc_t = kind == MGFVM_DIR_AMUF ? 1.0 / g.prsc : kind == MGFVM_DIR_PRSC ? -g.amuf / (g.prsc * g.prsc) : 0.0;
-    }
-    if (kind == MGFVM_DIR_INLET) {
-        std::vector<double> col(npy_of(g, 0), 0.0);
-        col[idx + 1] = 1.0;
+    const size_t at = x->tcase_off[c0], end = x->tcase_off[c0 + n - 1] + x->tcase_bytes[c0 + n - 1];
+    CK(cudaMemsetAsync(x->tpool + at, 0, end - at, x->stream));
+    for (int c = c0; c < c0 + n; ++c) {
+        const mgfvm_config &g = x->cfg[c];
+        const int kind = x->dir_kind[c];
         for (int ig = 0; ig < g.ngrid; ++ig) {
-            const int npx = npx_of(g, ig), npy = npy_of(g, ig);
-            if (ig > 0) {
-                std::vector<double> cc(npy, 0.0);
-                for (int jc = 1; jc <= npy - 2; ++jc) cc[jc] = 0.5 * (col[2 * jc] + col[2 * jc - 1]);
-                col.swap(cc);
-            }
-            CK(cudaMemcpy2DAsync(x->ht[c].lv[ig].t[S_U], sizeof(double) * npx, col.data(), sizeof(double),
-                                 sizeof(double), npy, cudaMemcpyHostToDevice, x->stream));
-            x->h2d += (long long)(sizeof(double) * npy);
+            LevelTan &D = x->ht[c].lv[ig];
+            D.amu_t = kind == MGFVM_DIR_AMUF ? 1.0 : 0.0;
+            D.amusc_t = kind == MGFVM_DIR_AMUF ? 1.0 / g.prsc : kind == MGFVM_DIR_PRSC ? -g.amuf / (g.prsc * g.prsc) : 0.0;
         }
+        x->ht[c].face = kind == MGFVM_DIR_INLET ? x->dir_index[c] : -1;
     }
-    CK(cudaMemcpyAsync(x->dt + c, &x->ht[c], sizeof(CaseTan), cudaMemcpyHostToDevice, x->stream));
-    x->h2d += (long long)sizeof(CaseTan);
+    CK(cudaMemcpyAsync(x->dt + c0, &x->ht[c0], sizeof(CaseTan) * n, cudaMemcpyHostToDevice, x->stream));
+    x->h2d += (long long)sizeof(CaseTan) * n;
+    const cudaError_t e = launch_seed_tangent(x->dc + c0, x->dt + c0, n, x->stream);
+    if (e != cudaSuccess) return mgfvm_fail(MGFVM_ECUDA, "seeding of directions: %s", cudaGetErrorString(e));
+    ++x->launches;
     CK(cudaStreamSynchronize(x->stream));
     return MGFVM_OK;
 }
@@ -1137,32 +1132,32 @@ int init_state(mgfvm_ctx *x, int only_case)
     cudaError_t e = launch_init(dc, di, n, x->maxng, x->maxcells.data(), max_obs, max_npy, x->stream);
     if (e != cudaSuccess) return mgfvm_fail(MGFVM_ECUDA, "init kernels: %s", cudaGetErrorString(e));
     x->launches += 3LL * x->maxng + 1 + (x->maxng - 1);
+    if (x->opt.tangent) return seed_tangent(x, only_case >= 0 ? only_case : 0, n);
     CK(cudaStreamSynchronize(x->stream));
-    if (x->opt.tangent)
-        for (int c = 0; c < x->ncases; ++c)
-            if (only_case < 0 || c == only_case) RC(seed_tangent(x, c));
     return MGFVM_OK;
 }
 
 int upload_profiles(mgfvm_ctx *x)
 {
-    size_t tot = 0;
-    for (auto &p : x->profile) tot += p.size();
-    if (x->dprofile) { ctx_free(x, x->dprofile); x->dprofile = nullptr; }
-    if (tot) {
-        CK(ctx_malloc(x, (void **)&x->dprofile, sizeof(double) * tot));
+    std::vector<double> all;
+    for (auto &p : x->profile) all.insert(all.end(), p.begin(), p.end());
+    if (all.size() > x->profile_cap) {
+        if (x->dprofile) ctx_free(x, x->dprofile);
+        x->dprofile = nullptr;
+        x->profile_cap = 0;
+        CK(ctx_malloc(x, (void **)&x->dprofile, sizeof(double) * all.size()));
+        x->profile_cap = all.size();
     }
     size_t off = 0;
     for (int c = 0; c < x->ncases; ++c) {
         auto &p = x->profile[c];
         x->hinit[c].profile = p.empty() ? nullptr : x->dprofile + off;
         x->hinit[c].nprofile = (int)p.size();
-        if (!p.empty()) CK(cudaMemcpy(x->dprofile + off, p.data(), sizeof(double) * p.size(), cudaMemcpyHostToDevice));
-        x->h2d += (long long)(sizeof(double) * p.size());
         off += p.size();
     }
+    if (!all.empty()) CK(cudaMemcpy(x->dprofile, all.data(), sizeof(double) * all.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(x->dinit, x->hinit.data(), sizeof(InitDev) * x->ncases, cudaMemcpyHostToDevice));
-    x->h2d += (long long)sizeof(InitDev) * x->ncases;
+    x->h2d += (long long)(sizeof(double) * all.size()) + (long long)sizeof(InitDev) * x->ncases;
     return MGFVM_OK;
 }
 
@@ -1247,11 +1242,21 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         for (int ig = 0; ig < x->cfg[c].ngrid; ++ig)
             x->maxcells[ig] = std::max(x->maxcells[ig], npx_of(x->cfg[c], ig) * npy_of(x->cfg[c], ig));
 
-    // obstacle programs (host)
+    // obstacle programs (host); a case whose grid and obstacles are those of the case before
+    // it (every direction of a gradient) uses that one's, here and on the device
     x->progs.assign((size_t)ncases * MAXLEV, mgfvm_obstacle_prog{});
-    for (int c = 0; c < ncases; ++c)
+    x->prog_case.resize(ncases);
+    auto same_obstacles = [&](int a, int b) {
+        const mgfvm_config &A = x->cfg[a], &B = x->cfg[b];
+        return A.nfx == B.nfx && A.nfy == B.nfy && A.ngrid == B.ngrid && A.ig_obs == B.ig_obs &&
+               A.ibeg_obs == B.ibeg_obs && x->obs[a] == x->obs[b];
+    };
+    for (int c = 0; c < ncases; ++c) {
+        x->prog_case[c] = c > 0 && same_obstacles(c - 1, c) ? x->prog_case[c - 1] : c;
+        if (x->prog_case[c] != c) continue;
         for (int ig = 0; ig < x->cfg[c].ngrid; ++ig)
             RC(mgfvm_build_obstacle_prog(&x->cfg[c], ig, &x->progs[(size_t)c * MAXLEV + ig]));
+    }
 
     CK(cudaSetDevice(x->device));
     CK(cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking));
@@ -1280,19 +1285,37 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
             const int ns = ig == 0 ? NSLOTS : NSLOTS_LEVEL;
             for (int s = 0; s < NSLOTS; ++s) p.slot[s] = s < ns ? take(n * sizeof(double)) : (size_t)-1;
             p.tag = take(n * sizeof(int));
-            const mgfvm_obstacle_prog &P = x->progs[(size_t)c * MAXLEV + ig];
-            p.seq = P.nseq ? take(n * sizeof(unsigned)) : (size_t)-1;
-            p.pdst = P.ncopy ? take(P.ncopy * sizeof(int)) : (size_t)-1;
-            p.psrc = P.ncopy ? take(P.ncopy * sizeof(int)) : (size_t)-1;
+            const mgfvm_obstacle_prog &P = x->prog(c, ig);
             p.pbuf = P.ncopy ? take(P.ncopy * sizeof(double)) : (size_t)-1;
-            const bool fan = P.ncopy && P.fan;
-            p.pcode = fan ? take(n * sizeof(int)) : (size_t)-1;
-            p.pfan = fan ? take(2 * (size_t)P.ncopy * sizeof(int)) : (size_t)-1;
             pend.push_back(p);
         }
         const long long n0 = (long long)(npx_of(g, 0) - 2) * (npy_of(g, 0) - 2);
         part_off[c] = take((size_t)std::max({nblk(n0), tiles_of(npx_of(g, 0) - 2, npy_of(g, 0) - 2), 64}) * RED_STRIDE * sizeof(double));
         cnt_off[c] = take(16 * sizeof(unsigned));
+    }
+    // the obstacle programs: what one case uploads lies together, one copy a case (an array
+    // a copy, 15 a case of three levels: 13 ms to create the 66 cases of a 64 x 64 gradient;
+    // one copy and shared programs: 1.7)
+    std::vector<size_t> prog_at(ncases), prog_end(ncases);
+    for (size_t k = 0, k0 = 0; k < pend.size(); ++k) {
+        Pend &p = pend[k];
+        if (p.ig == 0) k0 = k;
+        if (p.ig == 0) prog_at[p.c] = prog_end[p.c] = off = align_up(off, 256);
+        const int r = x->prog_case[p.c];
+        if (r != p.c) {   // (the case before it: the same levels)
+            const Pend &q = pend[k0 - x->cfg[p.c].ngrid + p.ig];
+            p.seq = q.seq; p.pdst = q.pdst; p.psrc = q.psrc; p.pcode = q.pcode; p.pfan = q.pfan;
+            continue;
+        }
+        const mgfvm_obstacle_prog &P = x->prog(p.c, p.ig);
+        const size_t n = (size_t)npx_of(x->cfg[p.c], p.ig) * npy_of(x->cfg[p.c], p.ig);
+        p.seq = P.nseq ? take(n * sizeof(unsigned)) : (size_t)-1;
+        p.pdst = P.ncopy ? take(P.ncopy * sizeof(int)) : (size_t)-1;
+        p.psrc = P.ncopy ? take(P.ncopy * sizeof(int)) : (size_t)-1;
+        const bool fan = P.ncopy && P.fan;
+        p.pcode = fan ? take(n * sizeof(int)) : (size_t)-1;
+        p.pfan = fan ? take(2 * (size_t)P.ncopy * sizeof(int)) : (size_t)-1;
+        prog_end[p.c] = off;
     }
     const size_t pool_bytes = align_up(off, 256);
     x->pool_bytes = pool_bytes;
@@ -1300,7 +1323,7 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
     if (me != cudaSuccess)
         return mgfvm_fail(me == cudaErrorMemoryAllocation ? MGFVM_ENOMEM : MGFVM_ECUDA,
                           "device pool of %zu bytes: %s", pool_bytes, cudaGetErrorString(me));
-    CK(cudaMemset(x->pool, 0, pool_bytes));
+    CK(cudaMemsetAsync(x->pool, 0, pool_bytes, x->stream));
 
     for (int c = 0; c < ncases; ++c) {
         CaseDev &C = x->hc[c];
@@ -1321,6 +1344,7 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         C.partials = (double *)(x->pool + part_off[c]);
         C.counters = (unsigned *)(x->pool + cnt_off[c]);
     }
+    std::vector<char> image;   // of one case's obstacle programs
     for (const Pend &p : pend) {
         CaseDev &C = x->hc[p.c];
         LevelDev &L = C.lv[p.ig];
@@ -1341,50 +1365,53 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         if (sb > 0xffffffffull) return mgfvm_fail(MGFVM_ENOMEM, "a level array of %zu bytes", sb);
         L.sb = (unsigned)sb;
         L.tag = (int *)(x->pool + p.tag);
-        const mgfvm_obstacle_prog &P = x->progs[(size_t)p.c * MAXLEV + p.ig];
+        const mgfvm_obstacle_prog &P = x->prog(p.c, p.ig);
         L.ncopy = P.ncopy;
         L.hazard = P.hazard;
-        L.seq = nullptr; L.pdst = nullptr; L.psrc = nullptr; L.pbuf = nullptr;
-        L.pcode = nullptr; L.pfan = nullptr;
+        L.seq = p.seq == (size_t)-1 ? nullptr : (unsigned *)(x->pool + p.seq);
+        L.pdst = p.pdst == (size_t)-1 ? nullptr : (int *)(x->pool + p.pdst);
+        L.psrc = p.psrc == (size_t)-1 ? nullptr : (int *)(x->pool + p.psrc);
+        L.pbuf = p.pbuf == (size_t)-1 ? nullptr : (double *)(x->pool + p.pbuf);
+        L.pcode = p.pcode == (size_t)-1 ? nullptr : (int *)(x->pool + p.pcode);
+        L.pfan = p.pfan == (size_t)-1 ? nullptr : (int *)(x->pool + p.pfan);
+        const size_t base = prog_at[p.c], bytes = prog_end[p.c] - base;
+        if (bytes == 0) continue;
+        if (p.ig == 0) image.assign(bytes, 0);
         if (P.nseq) {
-            const size_t n = (size_t)L.npx * L.npy;
-            std::vector<unsigned> dense(n, 0u);
+            unsigned *dense = (unsigned *)(image.data() + (p.seq - base));
             for (int k = 0; k < P.nseq; ++k) dense[P.cells[k]] = P.codes[k];
-            unsigned *d = (unsigned *)(x->pool + p.seq);
-            CK(cudaMemcpy(d, dense.data(), n * sizeof(unsigned), cudaMemcpyHostToDevice));
-            x->h2d += (long long)(n * sizeof(unsigned));
-            L.seq = d;
         }
         if (P.ncopy) {
-            int *dd = (int *)(x->pool + p.pdst), *ds = (int *)(x->pool + p.psrc);
-            CK(cudaMemcpy(dd, P.dst, P.ncopy * sizeof(int), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(ds, P.src, P.ncopy * sizeof(int), cudaMemcpyHostToDevice));
-            x->h2d += 2LL * P.ncopy * (long long)sizeof(int);
-            L.pdst = dd; L.psrc = ds;
-            L.pbuf = (double *)(x->pool + p.pbuf);
+            std::memcpy(image.data() + (p.pdst - base), P.dst, P.ncopy * sizeof(int));
+            std::memcpy(image.data() + (p.psrc - base), P.src, P.ncopy * sizeof(int));
         }
         if (p.pcode != (size_t)-1) {
             // per cell: PCODE_DST when the copy writes it, 1 + its first fan entry when
             // its update thread performs copies
-            const size_t n = (size_t)L.npx * L.npy;
-            std::vector<int> code(n, 0);
+            int *code = (int *)(image.data() + (p.pcode - base));
             for (int k = 0; k < P.ncopy; ++k) {
                 code[P.fan[2 * k] & ~PFAN_LAST] |= PCODE_DST;
                 if (k == 0 || P.owners[k] != P.owners[k - 1]) code[P.owners[k]] |= k + 1;
             }
-            int *dc = (int *)(x->pool + p.pcode), *df = (int *)(x->pool + p.pfan);
-            CK(cudaMemcpy(dc, code.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(df, P.fan, 2 * (size_t)P.ncopy * sizeof(int), cudaMemcpyHostToDevice));
-            x->h2d += (long long)(n + 2 * (size_t)P.ncopy) * (long long)sizeof(int);
-            L.pcode = dc;
-            L.pfan = df;
+            std::memcpy(image.data() + (p.pfan - base), P.fan, 2 * (size_t)P.ncopy * sizeof(int));
+        }
+        if (p.ig == g.ngrid - 1) {
+            CK(cudaMemcpyAsync(x->pool + base, image.data(), bytes, cudaMemcpyHostToDevice, x->stream));
+            x->h2d += (long long)bytes;
         }
     }
 
     // init parameters
     size_t nobs_tot = 0;
     for (int c = 0; c < ncases; ++c) nobs_tot += x->obs[c].size();
-    if (nobs_tot) CK(ctx_malloc(x, (void **)&x->dobs, sizeof(int) * nobs_tot));
+    std::vector<int> obs_all;
+    obs_all.reserve(nobs_tot);
+    for (int c = 0; c < ncases; ++c) obs_all.insert(obs_all.end(), x->obs[c].begin(), x->obs[c].end());
+    if (nobs_tot) {
+        CK(ctx_malloc(x, (void **)&x->dobs, sizeof(int) * nobs_tot));
+        CK(cudaMemcpyAsync(x->dobs, obs_all.data(), sizeof(int) * nobs_tot, cudaMemcpyHostToDevice, x->stream));
+        x->h2d += (long long)(sizeof(int) * nobs_tot);
+    }
     x->hinit.assign(ncases, InitDev{});
     size_t ooff = 0;
     for (int c = 0; c < ncases; ++c) {
@@ -1398,8 +1425,6 @@ int create_impl(const mgfvm_config *cases, int ncases, const mgfvm_options *opt_
         P.ig_obs = g.ig_obs; P.ibeg_obs = g.ibeg_obs; P.nobs = g.nobs;
         P.obs = nullptr;
         if (g.nobs) {
-            CK(cudaMemcpy(x->dobs + ooff, x->obs[c].data(), sizeof(int) * x->obs[c].size(), cudaMemcpyHostToDevice));
-            x->h2d += (long long)(sizeof(int) * x->obs[c].size());
             P.obs = x->dobs + ooff;
             ooff += x->obs[c].size();
         }
@@ -2120,6 +2145,19 @@ int mgfvm_objective(mgfvm_ctx *x, int icase, double *J, double *dJ)
     return MGFVM_OK;
 }
 
+// dJ of every case, summed on the device in objective_of's order (one number a case comes
+// back instead of two fields).
+static int all_tangent_objectives(mgfvm_ctx *x, double *dj)
+{
+    const cudaError_t e = launch_objective_tangent(x->dc, x->dt, x->ncases, x->stream);
+    if (e != cudaSuccess) return mgfvm_fail(MGFVM_ECUDA, "objective's derivative: %s", cudaGetErrorString(e));
+    CK(cudaStreamSynchronize(x->stream));
+    CK(cudaMemcpy2D(dj, sizeof(double), &x->dt->dj, sizeof(CaseTan), sizeof(double), x->ncases, cudaMemcpyDeviceToHost));
+    ++x->launches;
+    x->d2h += (long long)sizeof(double) * x->ncases;
+    return MGFVM_OK;
+}
+
 int mgfvm_gradient(const mgfvm_config *cfg, const double *inlet_u, int n_inlet, int ncycles, int device,
                    double *J, double *dJ_dinlet, double *dJ_damuf, double *dJ_dprsc)
 {
@@ -2160,10 +2198,12 @@ int mgfvm_gradient(const mgfvm_config *cfg, const double *inlet_u, int n_inlet, 
             if ((rc = init_state(x, -1)) != MGFVM_OK) break;
             if ((rc = mgfvm_cycle(x, ncycles)) != MGFVM_OK) break;
             if (d0 == 0 && J && (rc = mgfvm_objective(x, 0, J, nullptr)) != MGFVM_OK) break;
-            for (int c = 0; c < n && rc == MGFVM_OK; ++c) {
+            std::vector<double> dj(n);
+            if ((rc = all_tangent_objectives(x, dj.data())) != MGFVM_OK) break;
+            for (int c = 0; c < n; ++c) {
                 const int d = d0 + c;
                 double *dst = d < nf ? (dJ_dinlet ? dJ_dinlet + d : nullptr) : d == nf ? dJ_damuf : dJ_dprsc;
-                if (dst) rc = mgfvm_objective(x, c, nullptr, dst);
+                if (dst) *dst = dj[c];
             }
         } while (0);
         mgfvm_destroy(x);

@@ -66,7 +66,13 @@ struct LevelTan {
 };
 struct CaseTan {
     LevelTan lv[MAXLEV];
+    int face;   // the level-0 inlet face the case's direction moves (0-based), -1: none
+    double dj;  // k_objective_tangent's result
 };
+// mg_tangent.cu, of cases whose tables start at cs and ts: seed the inlet directions on
+// zeroed storage; the derivative of the objective, into dj.
+cudaError_t launch_seed_tangent(const CaseDev *cs, const CaseTan *ts, int n, cudaStream_t s);
+cudaError_t launch_objective_tangent(const CaseDev *cs, CaseTan *ts, int n, cudaStream_t s);
 
 struct Tan {
     using T = Dual;

@@ -29,11 +29,16 @@
 
 #define SEQ_MAX 14
 
-static int cmp_pair(const void *a, const void *b)
-{
-    const int *x = (const int *)a, *y = (const int *)b;
-    return (x[0] > y[0]) - (x[0] < y[0]);
-}
+/* Sets of cells, 64 to a word: the lists below are read off them in ascending order, for
+ * the few cells an obstacle touches, without a pass over the level (64 cases of 256 x 256
+ * with 20 obstacles each, all levels: 10 ms; by passes and sorts 51). */
+typedef unsigned long long cellset;
+#define ADD_CELL(set, q) ((set)[(q) >> 6] |= 1ull << ((q) & 63))
+#define HAS_CELL(set, q) (((set)[(q) >> 6] >> ((q) & 63)) & 1)
+#define EACH_CELL(set, words, q)                                                     \
+    for (size_t w_ = 0; w_ < (words); ++w_)                                          \
+        for (unsigned long long b_ = (set)[w_]; b_; b_ &= b_ - 1)                    \
+            for (int q = (int)(w_ * 64) + __builtin_ctzll(b_), once_ = 1; once_; once_ = 0)
 
 int mgfvm_build_obstacle_prog(const mgfvm_config *c, int ig, mgfvm_obstacle_prog *out)
 {
@@ -42,69 +47,72 @@ int mgfvm_build_obstacle_prog(const mgfvm_config *c, int ig, mgfvm_obstacle_prog
     int nx = c->nfx / (1 << ig) + 2, ny = c->nfy / (1 << ig) + 2;
     size_t n = (size_t)nx * ny;
     int *origin = (int *)malloc(sizeof(int) * n);
-    unsigned char *written = (unsigned char *)calloc(n, 1);
+    const size_t words = (n + 63) / 64;
+    cellset *sets = (cellset *)calloc(3 * words, sizeof(cellset));
+    cellset *written = sets, *added = sets + words, *owner = sets + 2 * words;
     unsigned *seq = (unsigned *)calloc(n, sizeof(unsigned));
-    if (!origin || !written || !seq) {
-        free(origin); free(written); free(seq);
+    if (!origin || !sets || !seq) {
+        free(origin); free(sets); free(seq);
         return mgfvm_fail(MGFVM_ENOMEM, "obstacle program: out of host memory");
     }
     for (size_t q = 0; q < n; ++q) origin[q] = (int)q;
 
-    int overflow = 0;
+    int overflow = 0, maxa = 0;
     for (int k = 0; k < c->nobs; ++k) {
         int r[4];
         mgfvm_obstacle_range(c, k, ig, r);
         int is = r[0], ie = r[1], js = r[2], je = r[3];
         /* pressure copies, in the reference's order */
-        for (int i = is; i <= ie; ++i) { int d = js * nx + i; origin[d] = origin[d - nx]; written[d] = 1; }
-        for (int i = is; i <= ie; ++i) { int d = je * nx + i; origin[d] = origin[d + nx]; written[d] = 1; }
-        for (int j = js; j <= je; ++j) { int d = j * nx + is; origin[d] = origin[d - 1]; written[d] = 1; }
-        for (int j = js; j <= je; ++j) { int d = j * nx + ie; origin[d] = origin[d + 1]; written[d] = 1; }
-        /* diffusion additions, i outer and j inner as in :941-962 */
-        for (int i = is; i <= ie; ++i)
-            for (int j = js; j <= je; ++j) {
-                int q = j * nx + i;
-                const int recv[4] = {q - 1, q + 1, q - nx, q + nx};
-                for (int t = 0; t < 4; ++t) {
-                    int x = recv[t], xi = x % nx, xj = x / nx;
-                    if (xi < 1 || xi > nx - 2 || xj < 1 || xj > ny - 2) continue;
-                    unsigned cnt = seq[x] >> 28;
-                    if (cnt >= SEQ_MAX) { overflow = 1; continue; }
-                    seq[x] = (seq[x] & 0x0FFFFFFFu) | ((unsigned)t << (2 * cnt)) | ((cnt + 1) << 28);
-                }
+        for (int i = is; i <= ie; ++i) { int d = js * nx + i; origin[d] = origin[d - nx]; ADD_CELL(written, d); }
+        for (int i = is; i <= ie; ++i) { int d = je * nx + i; origin[d] = origin[d + nx]; ADD_CELL(written, d); }
+        for (int j = js; j <= je; ++j) { int d = j * nx + is; origin[d] = origin[d - 1]; ADD_CELL(written, d); }
+        for (int j = js; j <= je; ++j) { int d = j * nx + ie; origin[d] = origin[d + 1]; ADD_CELL(written, d); }
+        /* diffusion additions, i outer and j inner as in :941-962: what a cell receives from
+         * this obstacle comes from its west, south, north, east neighbour, in that order */
+        if (ie < is || je < js) continue;
+        for (int j = js > 1 ? js - 1 : 1; j <= je + 1 && j <= ny - 2; ++j) {
+            const int in = j >= js && j <= je, lo = in ? is - 1 : is, hi = in ? ie + 1 : ie;
+            const int sn = j - 1 >= js && j - 1 <= je, nn = j + 1 >= js && j + 1 <= je;
+            for (int i = lo > 1 ? lo : 1; i <= hi && i <= nx - 2; ++i) {
+                const int x = j * nx + i, col = i >= is && i <= ie;
+                unsigned code = 0, k2 = 0;
+                if (in && i - 1 >= is && i - 1 <= ie) { code = 1; k2 = 2; }
+                if (sn && col) { code |= 3u << k2; k2 += 2; }
+                if (nn && col) { code |= 2u << k2; k2 += 2; }
+                if (in && i + 1 >= is && i + 1 <= ie) k2 += 2;
+                const unsigned s = seq[x], cnt = s >> 28, now = cnt + k2 / 2;
+                if (now > SEQ_MAX) { overflow = 1; continue; }
+                seq[x] = (s & 0x0FFFFFFFu) | (code << (2 * cnt)) | (now << 28);
+                if ((int)now > maxa) maxa = (int)now;
+                if (s == 0 && now) ADD_CELL(added, x);
             }
+        }
     }
     if (overflow) {
-        free(origin); free(written); free(seq);
+        free(origin); free(sets); free(seq);
         return mgfvm_fail(MGFVM_EUNSUPPORTED,
                           "level %d: a cell receives more than %d obstacle-face additions "
                           "(overlapping obstacles)", ig, SEQ_MAX);
     }
-    int ncopy = 0, nseq = 0, maxa = 0;
-    for (size_t q = 0; q < n; ++q) {
-        if (written[q] && origin[q] != (int)q) ++ncopy;
-        if (seq[q]) { ++nseq; int a = (int)(seq[q] >> 28); if (a > maxa) maxa = a; }
-    }
-    int *pairs = (int *)malloc(sizeof(int) * 2 * (size_t)(ncopy ? ncopy : 1));
+    int ncopy = 0, nseq = 0;
+    EACH_CELL(written, words, q) if (origin[q] != q) ++ncopy;
+    for (size_t w = 0; w < words; ++w) nseq += __builtin_popcountll(added[w]);
     out->dst = (int *)malloc(sizeof(int) * (size_t)(ncopy ? ncopy : 1));
     out->src = (int *)malloc(sizeof(int) * (size_t)(ncopy ? ncopy : 1));
     out->cells = (int *)malloc(sizeof(int) * (size_t)(nseq ? nseq : 1));
     out->codes = (unsigned *)malloc(sizeof(unsigned) * (size_t)(nseq ? nseq : 1));
-    if (!pairs || !out->dst || !out->src || !out->cells || !out->codes) {
-        free(pairs); free(origin); free(written); free(seq);
+    if (!out->dst || !out->src || !out->cells || !out->codes) {
+        free(origin); free(sets); free(seq);
         mgfvm_free_obstacle_prog(out);
         return mgfvm_fail(MGFVM_ENOMEM, "obstacle program: out of host memory");
     }
     int m = 0;
-    for (size_t q = 0; q < n; ++q)
-        if (written[q] && origin[q] != (int)q) { pairs[2 * m] = (int)q; pairs[2 * m + 1] = origin[q]; ++m; }
-    qsort(pairs, (size_t)m, 2 * sizeof(int), cmp_pair);
+    EACH_CELL(written, words, q)
+        if (origin[q] != q) { out->dst[m] = q; out->src[m] = origin[q]; ++m; }
     int hazard = 0, outlet = 0;
     for (int k = 0; k < m; ++k) {
-        out->dst[k] = pairs[2 * k];
-        out->src[k] = pairs[2 * k + 1];
         int s = out->src[k];
-        if (written[s] && origin[s] != s) hazard = 1;
+        if (HAS_CELL(written, s) && origin[s] != s) hazard = 1;
         if (out->dst[k] % nx >= nx - 2 || s % nx >= nx - 2) outlet = 1;
     }
     out->touches_outlet = outlet;
@@ -113,11 +121,11 @@ int mgfvm_build_obstacle_prog(const mgfvm_config *c, int ig, mgfvm_obstacle_prog
     if (!hazard && m > 0) {
         /* group the copies by owner: the source when interior, else the interior cell
          * next to it (sources are at most one cell outside an interior obstacle) */
-        int *tri = (int *)malloc(sizeof(int) * 3 * (size_t)m);
+        int *place = (int *)calloc(n, sizeof(int)), *own = (int *)malloc(sizeof(int) * (size_t)m);
         out->owners = (int *)malloc(sizeof(int) * (size_t)m);
         out->fan = (int *)malloc(sizeof(int) * 2 * (size_t)m);
-        if (!tri || !out->owners || !out->fan) {
-            free(tri); free(pairs); free(origin); free(written); free(seq);
+        if (!place || !own || !out->owners || !out->fan) {
+            free(place); free(own); free(origin); free(sets); free(seq);
             mgfvm_free_obstacle_prog(out);
             return mgfvm_fail(MGFVM_ENOMEM, "obstacle program: out of host memory");
         }
@@ -125,25 +133,27 @@ int mgfvm_build_obstacle_prog(const mgfvm_config *c, int ig, mgfvm_obstacle_prog
             const int s0 = out->src[k], si = s0 % nx, sj = s0 / nx;
             const int oi = si < 1 ? 1 : (si > nx - 2 ? nx - 2 : si);
             const int oj = sj < 1 ? 1 : (sj > ny - 2 ? ny - 2 : sj);
-            tri[3 * k] = oj * nx + oi;
-            tri[3 * k + 1] = out->dst[k];
-            tri[3 * k + 2] = (oi == si && oj == sj) ? -1 : s0;
+            own[k] = oj * nx + oi;
+            ++place[own[k]];
+            ADD_CELL(owner, own[k]);
         }
-        qsort(tri, (size_t)m, 3 * sizeof(int), cmp_pair);   /* by owner */
+        int at = 0;
+        EACH_CELL(owner, words, q) { const int c1 = place[q]; place[q] = at; at += c1; }   /* counting sort */
         for (int k = 0; k < m; ++k) {
-            out->owners[k] = tri[3 * k];
-            const int last = k == m - 1 || tri[3 * (k + 1)] != tri[3 * k];
-            out->fan[2 * k] = tri[3 * k + 1] | (last ? PFAN_LAST : 0);
-            out->fan[2 * k + 1] = tri[3 * k + 2];
+            const int to = place[own[k]]++;
+            out->owners[to] = own[k];
+            out->fan[2 * to] = out->dst[k];
+            out->fan[2 * to + 1] = own[k] == out->src[k] ? -1 : out->src[k];
         }
-        free(tri);
+        for (int k = 0; k < m; ++k)
+            if (k == m - 1 || out->owners[k + 1] != out->owners[k]) out->fan[2 * k] |= PFAN_LAST;
+        free(place); free(own);
     }
     m = 0;
-    for (size_t q = 0; q < n; ++q)
-        if (seq[q]) { out->cells[m] = (int)q; out->codes[m] = seq[q]; ++m; }
+    EACH_CELL(added, words, q) { out->cells[m] = q; out->codes[m] = seq[q]; ++m; }
     out->nseq = m;
     out->max_adds = maxa;
-    free(pairs); free(origin); free(written); free(seq);
+    free(origin); free(sets); free(seq);
     return MGFVM_OK;
 }
 
