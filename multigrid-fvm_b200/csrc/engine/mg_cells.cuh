@@ -447,15 +447,16 @@ __device__ __forceinline__ bool div_plain(double a, const Recip &R)
 // cache).  The compiled division takes a slow path for the dividends met here in earnest,
 // zeros (fields at rest) and tiny ones: a zero's quotient is q0, whose sign is the
 // division's, and a tiny one is divided after scaling by 2^600 (exact) and scaled back,
-// exact where the quotient is normal and a correctly signed zero where it is below half the
-// smallest subnormal.
+// exact where the quotient is normal.  A subnormal one is rounded a second time there, which
+// can only be wrong where the first rounding hit the middle of two subnormals: those (the
+// rest, exact, is half their spacing) are left to the compiled division.
 static __device__ __noinline__ double div_by_rare(double a, double b, double y)
 {
     if (__double2hiint(y) != 0) {
         if (a == 0.0) return a * y;
         if (fabs(a) < 0x1p-918) {
-            const double q = markstein(a * 0x1p600, Recip{b, y});
-            if (exponent_in<-422, 1023>(q) || fabs(q) < 0x1p-476) return q * 0x1p-600;
+            const double q = markstein(a * 0x1p600, Recip{b, y}), c = q * 0x1p-600;
+            if (fabs(fma(-c, 0x1p600, q)) != 0x1p-475) return c;
         }
     }
     return a / b;

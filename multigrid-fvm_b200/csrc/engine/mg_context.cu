@@ -96,6 +96,9 @@ struct mgfvm_ctx {
     // tensor maps of the V-cycle's TMA-staged smoother launches (host copy, device table)
     std::vector<SmoothMap> hmaps;
     SmoothMap *dmaps = nullptr;
+    // and the tiles of its K_SMOOTH_Q launches that have more of them than SMs
+    std::vector<QTile> htiles;
+    QTile *dtiles = nullptr;
     std::vector<int> tail0;                   // per case: first one-CTA-kernel level chosen at creation
     std::vector<void *> pooled;               // buffers taken from the device's memory pool
     // the last mgfvm_adjoint: per case J and its gradient (nfy inlet faces, amuf, prsc)
@@ -169,7 +172,31 @@ struct Builder {
     mgfvm_ctx *x;
     std::vector<Launch> *out;
     std::vector<SmoothMap> *maps = nullptr;               // where TMA-staged launches may be emitted
+    std::vector<QTile> *qtiles = nullptr;                 // where tables of tiles may be emitted
     std::map<std::tuple<int, int, int>, int> map_index{};   // (level, bw, bh) -> first map of its cases
+    // (level, mode, equations, tile) -> first tile and their number
+    std::map<std::tuple<int, int, int, int, int>, std::pair<int, int>> tile_index{};
+
+    // the tiles of tw x th cells of a smoothing of the equations in `mask`, every case's
+    std::pair<int, int> smooth_tiles(int ig, int mode, int mask, int tw, int th)
+    {
+        const auto key = std::make_tuple(ig, mode, mask, tw, th);
+        auto it = tile_index.find(key);
+        if (it != tile_index.end()) return it->second;
+        const int base = (int)qtiles->size();
+        for (int c = 0; c < x->ncases; ++c) {
+            if (!mode_active(x->hc[c], ig, mode)) continue;
+            const LevelDev &L = x->hc[c].lv[ig];
+            for (int e = 0; e < 4; ++e) {
+                if (!((mask >> e) & 1)) continue;
+                const int wi = L.npx - (e == EQ_U ? 3 : 2), wj = L.npy - (e == EQ_V ? 3 : 2);
+                for (int ty = 0; ty * th < wj; ++ty)
+                    for (int tx = 0; tx * tw < wi; ++tx)
+                        qtiles->push_back(QTile{(char *)L.f[0], L.sb, L.npx, L.npy, tx, ty, c, e});
+            }
+        }
+        return tile_index[key] = {base, (int)qtiles->size() - base};
+    }
 
     // index of the per-case tensor maps of a (level, box) shape, or -1 where some case's
     // level cannot be staged by TMA
@@ -297,8 +324,8 @@ struct Builder {
                (t == 2 || (band_default(G) && one_size(ig, mx, my)));
     }
     // The sizes of batch at which band visits of a G-CTA level are the faster ones.  FP64:
-    // only where a pair of CTAs holds the level (66^2 of a 256^2 case; 64 cases 2.59 ms per
-    // V-cycle against 2.64 with tiles, 32 cases 1.40 against 1.36; on 130^2 they cost 2.75).
+    // only where a pair of CTAs holds the level (66^2 of a 256^2 case: 64 cases 2.32 ms per
+    // V-cycle against 2.34 with tiles, 128 4.52 against 4.53, 32 1.28 against 1.24).
     // Mixed precision, whose tiles are FP32 and slower here: BAND_MIN_CASES.
     bool band_default(int G) const
     {
@@ -316,7 +343,7 @@ struct Builder {
     // launches, tile and tiles per case; false where k_smooth's tiles are expected to be
     // faster, or the tuning asks for those.  Expected times in microseconds, fitted to both
     // kernels on 1 to 64 cases of 64^2 to 1024^2: a round of CTAs over the SMs takes 4.9 +
-    // 0.37 a unit here and 5.0 + 0.19 there; the tiles here are larger, so large levels need
+    // 0.37 a unit here (3.5 + 0.37 after the first, k_smooth_qs) and 5.0 + 0.19 there; the tiles here are larger, so large levels need
     // half as many rounds, while a level of one round either way favours k_smooth's faster
     // units unless a single launch can take all of them.  (p' on two cases, 20 units: 256^2
     // 19.0 against 28.8 us, 128^2 17.7 against 14.4, 64^2 13.2 in one launch against 14.4.)
@@ -347,6 +374,10 @@ struct Builder {
             return (double)((n + SMS - 1) / SMS);
         };
         auto side = [](int n, int most) { return (n + (n + most - 1) / most - 1) / ((n + most - 1) / most); };
+        // a table of tiles (k_smooth_qs) wants every row a multiple of 16 bytes
+        bool even = true;
+        for (const mgfvm_config &c : x->cfg) even = even && (ig >= c.ngrid || npx_of(c, ig) % 2 == 0);
+        const double later = even ? 3.5 : 4.9;
         double t_best = 1e300, t_old = 1e300;
         int dummy;
         for (int c = 1; c <= units; ++c) {
@@ -355,7 +386,7 @@ struct Builder {
             const int mx = SMOOTH_Q_COLS - 2 * u - 1, my = SMOOTH_Q_ROWS - 2 * u - 1;
             if (mx >= MIN_TILE && my >= MIN_TILE) {
                 QPlan p{c, side(wi, mx), side(wj, my), 0};
-                const double t = c * (0.3 + rounds(p.tw, p.th, p.tiles) * (4.9 + 0.37 * u));
+                const double t = c * (0.3 + 4.9 - later + rounds(p.tw, p.th, p.tiles) * (later + 0.37 * u));
                 if (t < t_best) {
                     t_best = t;
                     best = p;
@@ -416,6 +447,13 @@ struct Builder {
         QPlan qp;
         if (smooth_q_plan(ig, neq, units, tmp_ok, qp)) {
             int u0 = 0;
+            // more tiles than SMs: CTAs that go through a table of them
+            const int hmax = (units + qp.chunks - 1) / qp.chunks, bw = (qp.tw + 2 * hmax + 2) & ~1, bh = qp.th + 2 * hmax + 1;
+            int mi = -1;
+            std::pair<int, int> tab{0, 0};
+            if (maps && qtiles && mode != M_OP && (long long)qp.tiles * x->ncases * neq > SMS &&
+                (mi = smooth_maps(ig, bw, bh)) >= 0)
+                tab = smooth_tiles(ig, mode, mask, qp.tw, qp.th);
             for (int c = 0; c < qp.chunks; ++c) {
                 const int nu = units / qp.chunks + (c < units % qp.chunks ? 1 : 0);
                 // a later launch reads its coefficients before waiting for the one before it
@@ -424,6 +462,13 @@ struct Builder {
                 L.bh = qp.th;
                 L.grid = dim3((unsigned)qp.tiles, x->ncases, neq);
                 L.block = SMOOTH_Q_THREADS;
+                if (mi >= 0 && tab.second > SMS) {
+                    L.map = mi;
+                    L.tile0 = tab.first;
+                    L.a4 = tab.second;
+                    L.box = bw << 16 | bh;
+                    L.grid = dim3(SMS);
+                }
                 u0 += nu;
             }
             if ((qp.chunks & 1) == 0) return false;
@@ -1077,38 +1122,51 @@ int seed_tangent(mgfvm_ctx *x, int c0, int n)
     return MGFVM_OK;
 }
 
-// The V-cycle's launch list, and the device table of tensor maps its TMA-staged
-// smoother launches read (without that table, those launches are plain tile launches).
+// The V-cycle's launch list, and the device tables its smoother launches read: tensor maps
+// and tiles (without them, those launches are plain tile launches).
 int build_cycle(mgfvm_ctx *x)
 {
     x->cyc.clear();
     x->hmaps.clear();
-    if (x->dmaps) {
+    x->htiles.clear();
+    if (x->dmaps || x->dtiles) {
         cudaStreamSynchronize(x->stream);
-        ctx_free(x, x->dmaps);
+        if (x->dmaps) ctx_free(x, x->dmaps);
+        if (x->dtiles) ctx_free(x, x->dtiles);
         x->dmaps = nullptr;
+        x->dtiles = nullptr;
     }
     {
-        Builder b{x, &x->cyc, &x->hmaps};
+        Builder b{x, &x->cyc, &x->hmaps, &x->htiles};
         b.cycle();
     }
-    if (x->hmaps.empty()) return MGFVM_OK;
-    cudaError_t e = ctx_malloc(x, (void **)&x->dmaps, sizeof(SmoothMap) * x->hmaps.size());
-    if (e == cudaSuccess)
-        e = cudaMemcpy(x->dmaps, x->hmaps.data(), sizeof(SmoothMap) * x->hmaps.size(), cudaMemcpyHostToDevice);
+    const size_t nm = sizeof(SmoothMap) * x->hmaps.size(), nt = sizeof(QTile) * x->htiles.size();
+    cudaError_t e = cudaSuccess;
+    if (nm) e = ctx_malloc(x, (void **)&x->dmaps, nm);
+    if (e == cudaSuccess && nt) e = ctx_malloc(x, (void **)&x->dtiles, nt);
+    if (e == cudaSuccess && nm) e = cudaMemcpy(x->dmaps, x->hmaps.data(), nm, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && nt) e = cudaMemcpy(x->dtiles, x->htiles.data(), nt, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (x->dmaps) ctx_free(x, x->dmaps);
+        if (x->dtiles) ctx_free(x, x->dtiles);
         x->dmaps = nullptr;
+        x->dtiles = nullptr;
         x->cyc.clear();
         x->hmaps.clear();
+        x->htiles.clear();
         Builder b{x, &x->cyc};
         b.cycle();
         return MGFVM_OK;
     }
-    x->h2d += (long long)(sizeof(SmoothMap) * x->hmaps.size());
-    for (Launch &L : x->cyc)
+    x->h2d += (long long)(nm + nt);
+    for (Launch &L : x->cyc) {
         if (L.kernel == K_SMOOTH_TMA) L.ptr = x->dmaps + L.map;
+        if (L.kernel == K_SMOOTH_Q && L.a4) {
+            L.ptr = x->dmaps + L.map;
+            L.tiles = x->dtiles + L.tile0;
+        }
+    }
     return MGFVM_OK;
 }
 
@@ -1171,6 +1229,7 @@ void destroy_all(mgfvm_ctx *x)
     if (x->pool) ctx_free(x, x->pool);
     if (x->tpool) ctx_free(x, x->tpool);
     if (x->dmaps) ctx_free(x, x->dmaps);
+    if (x->dtiles) ctx_free(x, x->dtiles);
     if (x->dt) ctx_free(x, x->dt);
     if (x->hist) ctx_free(x, x->hist);
     if (x->dprofile) ctx_free(x, x->dprofile);

@@ -1725,7 +1725,8 @@ int smooth_pairs_side(int units, int threads)
 
 cudaError_t configure_kernels()
 {
-    cudaError_t e = cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM_MAX);
+    cudaError_t e = configure_smooth_q();
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM_MAX);
     const void *tma[] = {(const void *)k_smooth_tma<MGFVM_JACOBI, SMOOTH_BLOCK>,
                          (const void *)k_smooth_tma<MGFVM_JACOBI, SMOOTH_BLOCK / 2>,
                          (const void *)k_smooth_tma<MGFVM_JACOBI, SMOOTH_BLOCK / 4>,

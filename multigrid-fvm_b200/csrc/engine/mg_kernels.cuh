@@ -50,8 +50,11 @@ struct Launch {
     int block;
     int smem;
     int bw, bh;        // K_SMOOTH_TMA: box width and height; K_SMOOTH_Q: tile
-    int map;           // K_SMOOTH_TMA: index of its first tensor-map pair in the schedule's table
-    const void *ptr;   // K_SMOOTH_TMA: that pair on the device (one per case)
+    int box;           // K_SMOOTH_Q by a table of a4 tiles: box width << 16 | height
+    int map;           // these: index of its first tensor-map pair in the schedule's table
+    int tile0;         // K_SMOOTH_Q by a table: index of its first tile in the schedule's
+    const void *ptr;   // that pair on the device (one per case)
+    const void *tiles; // that tile on the device
 };
 
 // The tensor maps of one case for a TMA-staged smoother launch: the level's slot
@@ -107,6 +110,14 @@ cudaError_t launch_tile(const Launch &L, const CaseDev *dcases, CaseState *dstat
 constexpr int SMOOTH_Q_COLS = 54, SMOOTH_Q_ROWS = 56, SMOOTH_Q_THREADS = 384;
 cudaError_t launch_smooth_q(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
 
+// A tile of a launch of it (more tiles than SMs: its CTAs go through a table of them): the
+// level's first array, stride and size, the tile's place, the case and the equation.
+struct alignas(16) QTile {
+    char *b;
+    unsigned sb;
+    int npx, npy, tx, ty, icase, e;
+};
+cudaError_t configure_smooth_q();
 // The same on a caller's own level (mgfvm_rbgs_f64): the expected time of its plan, and the
 // launches (`tmp` unused where chunks is 1).
 double raw_q_plan(int wi, int wj, int units, int &chunks, int &tw, int &th);

@@ -50,79 +50,71 @@ struct QIn {
     bool vec;   // a block row's two cells may be loaded together (16-byte aligned)
 };
 
-// Tile (tx, ty) of tw x th cells.  `enter` waits for the launches before and says whether
-// the case is still running.  EARLY: the coefficients are read before that.
-template <bool EARLY, class Enter>
-__device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx, int ty, int tw, int th, int u0, int nu,
-                                              Enter enter)
+// Tile (tx, ty) of tw x th cells with a halo of nu, and where in its region a thread's block
+// lies: its first cell, and whether the region has it.
+struct QTileAt {
+    int x0, y0, x1, y1, cx0, cy0, rx1, ry1, i, j;
+    bool mine;
+};
+__device__ __forceinline__ QTileAt tile_at(int dx1, int dy1, int tx, int ty, int tw, int th, int nu, int qx, int qy)
 {
-    __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
-    double *phi = smq + 2 * QX;   // a row of slack on either side
-    const int npx = in.npx, dx1 = in.dx1, dy1 = in.dy1, t = threadIdx.x;
-    const int x0 = 1 + tx * tw, y0 = 1 + ty * th;
-    const int x1 = min(x0 + tw - 1, dx1), y1 = min(y0 + th - 1, dy1);
-    const int cx0 = max(x0 - nu, 0) & ~1, cy0 = max(y0 - nu, 0) & ~1;
-    const int rx1 = min(x1 + nu, dx1 + 1), ry1 = min(y1 + nu, dy1 + 1);
-    const int qx = t % QX, qy = t / QX, i = cx0 + BX * qx, j = cy0 + BY * qy;
-    const bool mine = active && qy < QY && i <= rx1 && j <= ry1;
-    const int q0 = j * npx + i;
-    const bool vec = in.vec;
+    QTileAt T;
+    T.x0 = 1 + tx * tw;
+    T.y0 = 1 + ty * th;
+    T.x1 = min(T.x0 + tw - 1, dx1);
+    T.y1 = min(T.y0 + th - 1, dy1);
+    T.cx0 = max(T.x0 - nu, 0) & ~1;
+    T.cy0 = max(T.y0 - nu, 0) & ~1;
+    T.rx1 = min(T.x1 + nu, dx1 + 1);
+    T.ry1 = min(T.y1 + nu, dy1 + 1);
+    T.i = T.cx0 + BX * qx;
+    T.j = T.cy0 + BY * qy;
+    T.mine = qy < QY && T.i <= T.rx1 && T.j <= T.ry1;
+    return T;
+}
 
-    // cell (x, y) of the block: k[y][x] = aw .. an, su, b, y; v = field
+// A block's cells: cell (x, y) has k[y][x] of aw, ae, as, an, su, the diagonal b with its
+// reciprocal rc, and the field v.
+struct QBlock {
     double w[BY][BX], ea[BY][BX], so[BY][BX], no[BY][BX], su[BY][BX], b[BY][BX], rc[BY][BX], v[BY][BX];
+};
+__device__ __forceinline__ void clear_block(QBlock &B)
+{
 #pragma unroll
     for (int y = 0; y < BY; ++y)
 #pragma unroll
         for (int x = 0; x < BX; ++x) {
-            w[y][x] = ea[y][x] = so[y][x] = no[y][x] = v[y][x] = 0.0;
-            su[y][x] = b[y][x] = 1.0;
+            B.w[y][x] = B.ea[y][x] = B.so[y][x] = B.no[y][x] = B.v[y][x] = 0.0;
+            B.su[y][x] = B.b[y][x] = 1.0;
         }
-    auto load = [&](const double *p, double (&a)[BY][BX]) {
-#pragma unroll
-        for (int y = 0; y < BY; ++y)
-            if (mine && j + y <= ry1) {
-                const double *g = p + q0 + y * npx;
-                if (vec) {
-                    const double2 d = *reinterpret_cast<const double2 *>(g);
-                    a[y][0] = d.x;
-                    a[y][1] = d.y;
-                } else {
-                    a[y][0] = g[0];
-                    if (i + 1 < npx) a[y][1] = g[1];
-                }
-            }
-    };
-    auto coefs = [&]() {
-        load(in.co[CK_AP], b);
-        load(in.co[CK_AW], w);
-        load(in.co[CK_AE], ea);
-        load(in.co[CK_AS], so);
-        load(in.co[CK_AN], no);
-        load(in.co[CK_SU], su);
-    };
-    if (EARLY) coefs();
-    const bool live = enter();
-    if (!active) return;
-    load(in.src, v);
-    if (!EARLY) coefs();
-    if (!live) return;
-    // cells outside the domain (the boundary ring, unused halo) are never updated; harmless
-    // operands keep their dead updates on the division's fast path
+}
+// The reciprocals, and the field into shared memory.  Cells outside the domain (the boundary
+// ring, unused halo) are never updated; harmless operands keep their dead updates on the
+// division's fast path.
+__device__ __forceinline__ void prepare_block(QBlock &B, const QTileAt &T, int dx1, int dy1, double *phi, int qx, int qy)
+{
 #pragma unroll
     for (int y = 0; y < BY; ++y)
 #pragma unroll
         for (int x = 0; x < BX; ++x) {
-            const bool dom = mine && i + x >= 1 && i + x <= dx1 && j + y >= 1 && j + y <= dy1 && i + x <= rx1 && j + y <= ry1;
-            if (!dom) b[y][x] = su[y][x] = 1.0;
-            rc[y][x] = make_recip(b[y][x]).y;
+            const bool dom = T.mine && T.i + x >= 1 && T.i + x <= dx1 && T.j + y >= 1 && T.j + y <= dy1 &&
+                             T.i + x <= T.rx1 && T.j + y <= T.ry1;
+            if (!dom) B.b[y][x] = B.su[y][x] = 1.0;
+            B.rc[y][x] = make_recip(B.b[y][x]).y;
         }
     if (qy < QY) {
 #pragma unroll
         for (int y = 0; y < BY; ++y)
 #pragma unroll
-            for (int x = 0; x < BX; ++x) phi[sh(BY * qy + y, x, qx)] = v[y][x];
+            for (int x = 0; x < BX; ++x) phi[sh(BY * qy + y, x, qx)] = B.v[y][x];
     }
-    __syncthreads();
+}
+// The units u0 .. u0 + nu - 1 (each between barriers; one precedes the first), then the tile,
+// plus the boundary ring where it touches it, to dst.
+__device__ __forceinline__ void smooth_block(QBlock &B, const QTileAt &T, int dx1, int dy1, int npx, double *phi, int qx,
+                                             int qy, int u0, int nu, double *dst)
+{
+    const int i = T.i, j = T.j, x0 = T.x0, x1 = T.x1, y0 = T.y0, y1 = T.y1;
     for (int h = 1; h <= nu; ++h) {
         const int g = nu - h;
         const int xl = max(1, x0 - g), xr = min(dx1, x1 + g), yl = max(1, y0 - g), yr = min(dy1, y1 + g);
@@ -140,12 +132,12 @@ __device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx
 #pragma unroll
             for (int y = 0; y < BY; ++y) {
                 const int x = (y + COL) & 1, r = BY * qy + y;
-                const double pw = x == 0 ? phi[sh(r, 1, qx - 1)] : v[y][0];
-                const double pe = x == 1 ? phi[sh(r, 0, qx + 1)] : v[y][1];
-                const double ps = y == 0 ? phi[sh(r - 1, x, qx)] : v[y - 1][x];
-                const double pn = y == BY - 1 ? phi[sh(r + 1, x, qx)] : v[y + 1][x];
-                const Recip R{b[y][x], rc[y][x]};
-                a[y] = (w[y][x] * pw + ea[y][x] * pe + so[y][x] * ps + no[y][x] * pn) + su[y][x];
+                const double pw = x == 0 ? phi[sh(r, 1, qx - 1)] : B.v[y][0];
+                const double pe = x == 1 ? phi[sh(r, 0, qx + 1)] : B.v[y][1];
+                const double ps = y == 0 ? phi[sh(r - 1, x, qx)] : B.v[y - 1][x];
+                const double pn = y == BY - 1 ? phi[sh(r + 1, x, qx)] : B.v[y + 1][x];
+                const Recip R{B.b[y][x], B.rc[y][x]};
+                a[y] = (B.w[y][x] * pw + B.ea[y][x] * pe + B.so[y][x] * ps + B.no[y][x] * pn) + B.su[y][x];
                 z[y] = markstein(a[y], R);
                 plain &= div_plain(a[y], R);
             }
@@ -153,14 +145,14 @@ __device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx
 #pragma unroll
                 for (int y = 0; y < BY; ++y) {
                     const int x = (y + COL) & 1;
-                    if (!div_plain(a[y], Recip{b[y][x], rc[y][x]})) z[y] = div_by_rare(a[y], b[y][x], rc[y][x]);
+                    if (!div_plain(a[y], Recip{B.b[y][x], B.rc[y][x]})) z[y] = div_by_rare(a[y], B.b[y][x], B.rc[y][x]);
                 }
             }
 #pragma unroll
             for (int y = 0; y < BY; ++y) {
                 const int x = (y + COL) & 1;
                 if (ax[x] && ay[y]) {
-                    v[y][x] = z[y];
+                    B.v[y][x] = z[y];
                     phi[sh(BY * qy + y, x, qx)] = z[y];
                 }
             }
@@ -169,19 +161,199 @@ __device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx
         else unit(std::integral_constant<int, 1>{});
         __syncthreads();
     }
-    // the tile, plus the boundary ring where it touches it
     const int ox0 = x0 == 1 ? 0 : x0, ox1 = x1 == dx1 ? x1 + 1 : x1;
     const int oy0 = y0 == 1 ? 0 : y0, oy1 = y1 == dy1 ? y1 + 1 : y1;
-    if (mine) {
+    if (T.mine) {
 #pragma unroll
         for (int y = 0; y < BY; ++y)
 #pragma unroll
             for (int x = 0; x < BX; ++x)
-                if (i + x >= ox0 && i + x <= ox1 && j + y >= oy0 && j + y <= oy1) in.dst[q0 + y * npx + x] = v[y][x];
+                if (i + x >= ox0 && i + x <= ox1 && j + y >= oy0 && j + y <= oy1) dst[(j + y) * npx + i + x] = B.v[y][x];
     }
 }
 
+// Tile (tx, ty) of a CTA that takes one.  `enter` waits for the launches before and says
+// whether the case is still running.  EARLY: the coefficients are read before that.
+template <bool EARLY, class Enter>
+__device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx, int ty, int tw, int th, int u0, int nu,
+                                              Enter enter)
+{
+    __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
+    double *phi = smq + 2 * QX;   // a row of slack on either side
+    const int npx = in.npx, t = threadIdx.x, qx = t % QX, qy = t / QX;
+    const QTileAt T = tile_at(in.dx1, in.dy1, tx, ty, tw, th, nu, qx, qy);
+    const int q0 = T.j * npx + T.i;
+    QBlock B;
+    clear_block(B);
+    auto load = [&](const double *p, double (&a)[BY][BX]) {
+#pragma unroll
+        for (int y = 0; y < BY; ++y)
+            if (active && T.mine && T.j + y <= T.ry1) {
+                const double *g = p + q0 + y * npx;
+                if (in.vec) {
+                    const double2 d = *reinterpret_cast<const double2 *>(g);
+                    a[y][0] = d.x;
+                    a[y][1] = d.y;
+                } else {
+                    a[y][0] = g[0];
+                    if (T.i + 1 < npx) a[y][1] = g[1];
+                }
+            }
+    };
+    auto coefs = [&]() {
+        load(in.co[CK_AP], B.b);
+        load(in.co[CK_AW], B.w);
+        load(in.co[CK_AE], B.ea);
+        load(in.co[CK_AS], B.so);
+        load(in.co[CK_AN], B.no);
+        load(in.co[CK_SU], B.su);
+    };
+    if (EARLY) coefs();
+    const bool live = enter();
+    if (!active) return;
+    load(in.src, B.v);
+    if (!EARLY) coefs();
+    if (!live) return;
+    prepare_block(B, T, in.dx1, in.dy1, phi, qx, qy);
+    __syncthreads();
+    smooth_block(B, T, in.dx1, in.dy1, npx, phi, qx, qy, u0, nu, in.dst);
+}
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Wait for the mbarrier's phase of parity `par` with at most `polls` polls; false on timeout.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned par, int polls)
+{
+    for (int it = 0; it < polls; ++it) {
+        unsigned done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(par)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void copy_box(void *to, const CUtensorMap *map, int x, int y, int slot, unsigned bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_addr(to)), "l"(map), "r"(x), "r"(y), "r"(slot), "r"(bar)
+                 : "memory");
+}
+
+// where the field lies after the coefficients of a box (a copy lands on a 128-byte boundary)
+__host__ __device__ constexpr int ahead_field(int box) { return (NCOEF * box + 15) & ~15; }
+
+__device__ __forceinline__ void copy_async16(void *to, const void *from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(to)), "l"(from) : "memory");
+}
+
 }  // namespace
+
+// The tiles of a launch that has more of them than SMs, by a CTA an SM that takes every
+// gridDim.x-th of the table `tab`.  While a tile is smoothed, one thread has the next one's
+// coefficients and field copied (TMA) into shared memory, from where the threads fetch their
+// blocks, and the table entry after that: only the first tile's way from memory is waited
+// for.  `maps` has each case's two tensor maps with a box of bw x bh cells (even bw: a box
+// starts at an even column).  A copy that does not land within `polls` polls:
+// CASE_WAIT_TIMEOUT, as k_smooth_tma.
+// A tile takes 3.5 us and 0.37 a unit here, 4.9 and 0.37 with a CTA a tile (k_smooth_q),
+// bound by the copies (25 MB a round of CTAs) and the fetch that waits for them.  Level 0 of
+// 64 256^2 obstacle cases: five p' units 88 us against 111, four of u, v, sc 225 against 300;
+// a V-cycle 2.36 ms against 2.60, of 8 cases 0.447 against 0.454.  (Copies by every thread,
+// cp.async, were no faster than none ahead: issuing them holds up the units' accesses.  Tiles
+// drawn from a counter: two ahead, so that the draw is not waited for, they balance no better.)
+template <bool EARLY>
+__global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
+    k_smooth_qs(const QTile *__restrict__ tab, int ntab, const SmoothMap *__restrict__ maps, CaseState *st,
+                int u0, int nu, int dir, int tw, int th, int bw, int bh, int polls)
+{
+    extern __shared__ __align__(128) double ahead[];   // coefficients, then the field
+    __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
+    __shared__ QTile entry[3];   // of tile k (its number in this CTA), in k % 3
+    __shared__ int there[3];     // there is a tile k
+    __shared__ __align__(8) unsigned long long mbar;
+    double *phi = smq + 2 * QX;
+    const int t = threadIdx.x, qx = t % QX, qy = t / QX, box = bw * bh, fbox = ahead_field(box);
+    const unsigned bar = smem_addr(&mbar);
+    auto fetch = [&](int k, int n) {   // the entry of tile k, number n
+        there[k % 3] = n < ntab;
+        if (n >= ntab) return;
+        for (int c = 0; c < (int)sizeof(QTile) / 16; ++c)
+            copy_async16(reinterpret_cast<char *>(&entry[k % 3]) + 16 * c, reinterpret_cast<const char *>(tab + n) + 16 * c);
+    };
+    auto first_cell = [&](int n0, int n) { return max(1 + n0 * n - nu, 0) & ~1; };
+    auto coefs = [&](const QTile &N) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     ::"r"(bar), "r"((unsigned)((NCOEF + 1) * box * sizeof(double)))
+                     : "memory");
+        copy_box(ahead, &maps[N.icase].coef, first_cell(N.tx, tw), first_cell(N.ty, th), co_slot(N.e, CK_AW), bar);
+    };
+    auto field = [&](const QTile &N) {
+        copy_box(ahead + fbox, &maps[N.icase].field, first_cell(N.tx, tw), first_cell(N.ty, th),
+                 dir == 1 ? eq_tmp(N.e) : eq_field(N.e), bar);
+    };
+    if (t == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        entry[0] = tab[blockIdx.x];
+        if (EARLY) coefs(entry[0]);
+        fetch(1, blockIdx.x + gridDim.x);
+    }
+    pdl_enter();
+    if (t == 0) {
+        if (!EARLY) coefs(entry[0]);
+        field(entry[0]);
+    }
+    __syncthreads();
+    for (int k = 0;; ++k) {
+        const QTile now = entry[k % 3];
+        const int dx1 = now.npx - (now.e == EQ_U ? 3 : 2), dy1 = now.npy - (now.e == EQ_V ? 3 : 2);
+        const QTileAt T = tile_at(dx1, dy1, now.tx, now.ty, tw, th, nu, qx, qy);
+        const bool live = !st[now.icase].done;
+        QBlock B;
+        clear_block(B);
+        const bool landed = mbar_wait(bar, k & 1, polls);
+        auto load = [&](int at, double (&a)[BY][BX]) {
+#pragma unroll
+            for (int y = 0; y < BY; ++y)
+                if (T.mine && T.j + y <= T.ry1) {
+                    const double2 d = *reinterpret_cast<const double2 *>(ahead + at + (BY * qy + y) * bw + BX * qx);
+                    a[y][0] = d.x;
+                    a[y][1] = d.y;
+                }
+        };
+        load(CK_AP * box, B.b);
+        load(CK_AW * box, B.w);
+        load(CK_AE * box, B.ea);
+        load(CK_AS * box, B.so);
+        load(CK_AN * box, B.no);
+        load(CK_SU * box, B.su);
+        load(fbox, B.v);
+        prepare_block(B, T, dx1, dy1, phi, qx, qy);
+        if (t == 0) asm volatile("cp.async.wait_all;" ::: "memory");   // entry k + 1
+        // one decision for the whole block; after it, `ahead` has been read
+        if (!__syncthreads_and(landed)) {
+            if (t == 0) atomicOr(&st[now.icase].status, (int)CASE_WAIT_TIMEOUT);
+            mbar_wait(bar, k & 1, TMA_WAIT_POLLS);
+            return;
+        }
+        const bool more = there[(k + 1) % 3];
+        if (t == 0 && more) {
+            coefs(entry[(k + 1) % 3]);
+            field(entry[(k + 1) % 3]);
+            fetch(k + 2, blockIdx.x + (k + 2) * gridDim.x);
+        }
+        if (live)
+            smooth_block(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
+                         reinterpret_cast<double *>(now.b + (unsigned long long)(unsigned)(dir == 0 ? eq_tmp(now.e) : eq_field(now.e)) * now.sb));
+        else
+            __syncthreads();   // (phi has been read before it is written again)
+        if (!more) return;
+    }
+}
 
 // blockIdx.x: tile, .y: case, .z: equation of `mask`; `dir` 0: from the field to the
 // equation's ping-pong buffer, 1: the reverse.  EARLY: a later launch of the smoothing.
@@ -222,8 +394,25 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1) r_smooth_q(QIn in, int u0
     });
 }
 
+cudaError_t configure_smooth_q()
+{
+    cudaError_t e = cudaSuccess;
+    for (const void *k : {(const void *)k_smooth_qs<false>, (const void *)k_smooth_qs<true>})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (ahead_field(SMOOTH_Q_COLS * SMOOTH_Q_ROWS) + SMOOTH_Q_COLS * SMOOTH_Q_ROWS) * (int)sizeof(double));
+    return e;
+}
+
 cudaError_t launch_smooth_q(const Launch &X, const CaseDev *dc, CaseState *ds, const Sched &S, cudaStream_t st)
 {
+    if (X.a4) {
+        const int bw = X.box >> 16, bh = X.box & 0xffff;
+        if (!X.ptr || !X.tiles || bw > SMOOTH_Q_COLS || bh > SMOOTH_Q_ROWS) return cudaErrorInvalidValue;
+        return launch_k(S.pdl, (X.a3 & 4) ? k_smooth_qs<true> : k_smooth_qs<false>, X.grid, SMOOTH_Q_THREADS,
+                        (ahead_field(bw * bh) + bw * bh) * (int)sizeof(double), st, (const QTile *)X.tiles, X.a4,
+                        (const SmoothMap *)X.ptr, ds, X.a1, X.a2, X.a3 & 3, X.bw, X.bh, bw, bh, S.tma_wait_polls);
+    }
     if (X.a3 & 4)
         return launch_k(S.pdl, k_smooth_q<true>, X.grid, SMOOTH_Q_THREADS, 0, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2,
                         X.a3 & 3, X.bw, X.bh);
