@@ -647,7 +647,7 @@ struct Builder {
             L.a4 = std::max(mu, 0);
             L.grid = dim3(visit ? 3 : 1, x->ncases);
             L.block = round32(mx * ((my + 1) / 2));
-            L.smem = (isolve == MGFVM_JACOBI ? 2 : 1) * mx * my * (int)sizeof(double);
+            L.smem = ((isolve == MGFVM_JACOBI ? 2 : 1) + (!visit ? 0 : what ? 5 : 1)) * mx * my * (int)sizeof(double);
             return;
         }
         int G, blk, smem;

@@ -878,39 +878,295 @@ __device__ __forceinline__ void cluster_barrier()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// A whole visit to a level that one CTA per case holds, as one launch of a cluster of
-// three CTAs per case (cluster rank r = blockIdx.x: u, v, sc).  CTA r runs its part of
-// the level's assembly `what` (the slices of k_asm with three slices: fluxes + u, v,
-// sc + outflow ghost) over every cell, then — once the whole cluster has assembled, as
-// the smoothers read nothing the other parts write — `mu` units of its equation in
-// place; after a second cluster barrier CTA 0 runs solve_pprime and update
-// (pp_level_body).  No thread leaves before the barriers: the case's activity is the
-// same for the three CTAs and only guards the work.
+// the shared::cluster address `p` (a shared-memory location of this CTA) has in CTA `rank`
+__device__ __forceinline__ unsigned cl_map(const void *p, unsigned rank)
+{
+    unsigned a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+// store v at the shared-memory location `p` has in CTA `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double *p, unsigned rank, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cl_map(p, rank)), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// A level's shared arrays, row after row, as tile_coef_* read them.
+struct Rows {
+    double *p;
+    int w;
+    __device__ __forceinline__ double *operator[](int y) const { return p + y * w; }
+};
+struct LevelGeo {
+    Rows cx, cy, qx, qy;
+};
+
+// The units 1 .. n of a level in shared memory (phi; Jacobi's second buffer phi2): a thread's
+// red cell 0 and black cell 1 at k with coefficients c, reciprocals R, in the domain where
+// `in`.  Barriers before and after.  Returns the buffer that holds the result.
 template <int ISOLVE>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SMOOTH_BLOCK, 1)
+__device__ __forceinline__ const double *level_units(const double (&c)[2][NCOEF], const Recip (&R)[2], const bool (&in)[2],
+                                                     const int (&k)[2], int n, int W, double *phi, double *phi2)
+{
+    for (int h = 1; h <= n; ++h) {
+        const double *cur = ISOLVE == MGFVM_JACOBI && ((h - 1) & 1) ? phi2 : phi;
+        double *nxt = ISOLVE == MGFVM_JACOBI && ((h - 1) & 1) ? phi : ISOLVE == MGFVM_JACOBI ? phi2 : phi;
+        if (ISOLVE == MGFVM_JACOBI) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+                if (in[x]) {
+                    const int q = k[x];
+                    nxt[q] = jacobi_value_r(c[x][0], c[x][1], c[x][2], c[x][3], R[x], c[x][5], cur[q - 1], cur[q + 1],
+                                            cur[q - W], cur[q + W], cur[q]);
+                }
+        } else if ((h & 1) ? in[0] : in[1]) {
+            const int q = (h & 1) ? k[0] : k[1];
+            const double(&a)[NCOEF] = (h & 1) ? c[0] : c[1];
+            nxt[q] = gs_value_r(a[0], a[1], a[2], a[3], (h & 1) ? R[0] : R[1], a[5], cur[q - 1], cur[q + 1], cur[q - W], cur[q + W]);
+        }
+        __syncthreads();
+    }
+    return ISOLVE == MGFVM_JACOBI && (n & 1) ? phi2 : phi;
+}
+
+// u, v of a visit's p' sources: from shared memory, with the cell's own face areas.
+struct VisitVel {
+    using T = double;
+    const FastLevel &L;
+    const double *u, *v;
+    double ax, ay;
+    __device__ __forceinline__ double ld(int s, int q) const { return s == S_U ? u[q] : v[q]; }
+    __device__ __forceinline__ double g(int s, int) const { return s == S_AREAX ? ax : ay; }
+};
+
+// A whole visit to a level that one CTA per case holds, as one launch of a cluster of
+// three CTAs per case (cluster rank r = blockIdx.x: u, v, sc).  A thread owns a vertical pair
+// of the padded level's cells throughout.  CTA r forms its equation's coefficients (`what`
+// not 0; else a restriction's launch has) from fluxes and conductances in shared memory, as
+// k_tile_asm, keeps them in registers and runs `mu` units in shared memory; it arrives at
+// the cluster's first barrier when it has read what the other two smooth and waits there
+// before it writes its field back (CTA 1 also into CTA 0's shared memory).  CTA 0 reads and
+// forms all it can of solve_pprime and update before the second barrier, after which u and v
+// are there, and runs them as pp_level_body.  Every thread takes both barriers: the case's
+// activity is the same for the three CTAs and only guards the work.
+// Bound by latency; it waits once each for the level's description (before the launch before
+// has finished), the fields, apu and apv, the barriers; then a p' half-sweep takes 0.2-0.3 us,
+// a Jacobi sweep 0.5 (FP64 pipe).  EARLY: update's operands are read before the units too
+// (blocks that leave a thread 96 registers).  A V-cycle of one 64^2 channel (two levels of
+// visits, Jacobi) 94 us against 102 with the assembly in global memory and every phase's
+// operands read when it began, of two 256^2 cases 244 against 259.
+template <int ISOLVE, int NT>
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
     k_level_visit(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int nu, int reduce, int fuse,
                   int what, int mu)
 {
-    pdl_enter();
+    constexpr bool JAC = ISOLVE == MGFVM_JACOBI, EARLY = NT < SMOOTH_BLOCK;
     extern __shared__ double sm[];
     const CaseDev &C = cs[blockIdx.y];
     CaseState &ST = st[blockIdx.y];
-    const bool active = case_active(C, ST, ig, mode);
-    const LevelDev &L = C.lv[ig];
-    const int r = blockIdx.x;
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
+    const bool on = mode_active(C, ig, mode);
+    const int W = L.npx, H = L.npy, n = W * H, r = blockIdx.x, t = threadIdx.x;
+    const int e = r == 0 ? EQ_U : r == 1 ? EQ_V : EQ_SC, field = eq_field(e);
+    const int i = t % W, j0 = 2 * (t / W);
+    const int j[2] = {((i + j0) & 1) == 0 ? j0 : j0 + 1, ((i + j0) & 1) == 0 ? j0 + 1 : j0};
+    const int k[2] = {j[0] * W + i, j[1] * W + i};
+    bool has[2], inner[2], in[2];   // a cell of the padded level, of its interior, of the equation's domain
+    double ax[2] = {0.0, 0.0}, ay[2] = {0.0, 0.0}, sp[2] = {0.0, 0.0};
+    unsigned code[2] = {0u, 0u};
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        has[x] = on && j[x] < H;
+        inner[x] = has[x] && i >= 1 && i <= W - 2 && j[x] >= 1 && j[x] <= H - 2;
+        in[x] = inner[x] && (r != 0 || i <= W - 3) && (r != 1 || j[x] <= H - 3);
+        if ((what || r == 0) && has[x]) {   // (nothing writes these)
+            ax[x] = io.g(S_AREAX, k[x]);
+            ay[x] = io.g(S_AREAY, k[x]);
+            if (what && in[x]) sp[x] = io.g(r == 0 ? S_SPU : r == 1 ? S_SPV : S_SPSC, k[x]);
+            if (r == 2 && in[x] && L.seq) code[x] = L.seq[k[x]];
+        }
+    }
+    double *phi = sm, *phi2 = sm + n, *vel = sm + (JAC ? 2 : 1) * n, *geo = vel + n;   // vel: CTA 0's v
+    if (!what) cluster_arrive();   // (CTA 0 is there to be written to)
+    pdl_enter();
+    const bool active = on && !ST.done;
+    double c[2][NCOEF], v[2] = {0.0, 0.0};
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        c[x][0] = c[x][1] = c[x][2] = c[x][3] = c[x][5] = 0.0;
+        c[x][4] = 1.0;
+    }
     if (what) {
         if (active) {
-            const unsigned w = asm_slice((unsigned)what, r, 3);
-            const int n = L.npx * L.npy;
-            for (int q = threadIdx.x; q < n; q += blockDim.x) cell_asm(L, C, FluxLive(L), q % L.npx, q / L.npx, w);
+            const LevelGeo g{{geo, W}, {geo + n, W}, {geo + 2 * n, W}, {geo + 3 * n, W}};
+            const bool ghost = r == 2 && (what & A_SC_OUTFLOW) && C.ibc_xp == 4 && i == W - 1;
+            double u[2] = {0.0, 0.0}, w[2] = {0.0, 0.0}, dp[2] = {0.0, 0.0}, res[2] = {0.0, 0.0};
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (has[x]) {
+                    u[x] = io.ld(S_U, k[x]);
+                    w[x] = io.ld(S_V, k[x]);
+                    if (r == 2) v[x] = io.ld(S_SC, ghost ? k[x] - 1 : k[x]);
+                }
+                if (in[x]) {
+                    if (r < 2) dp[x] = io.ld(S_P, k[x]) - io.ld(S_P, r == 0 ? k[x] + 1 : k[x] + W);
+                    res[x] = io.ld(r == 0 ? S_RESU : r == 1 ? S_RESV : S_RESSC, k[x]);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+                if (has[x]) {
+                    const double cx = 0.5 * u[x] * ax[x], cy = 0.5 * w[x] * ay[x];
+                    g.cx.p[k[x]] = cx;
+                    g.cy.p[k[x]] = cy;
+                    g.qx.p[k[x]] = div_by(ax[x], Recip{L.dx, L.rdx});
+                    g.qy.p[k[x]] = div_by(ay[x], Recip{L.dy, L.rdy});
+                    if (r == 0 && i <= W - 2 && j[x] <= H - 2) {
+                        io.st(S_CX, k[x], cx);
+                        io.st(S_CY, k[x], cy);
+                    }
+                    if (ghost) io.st(S_SC, k[x], v[x]);
+                    if (r < 2) v[x] = r == 0 ? u[x] : w[x];
+                }
+            __syncthreads();
+            const Recip rm{C.relxm, C.rrelxm};
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (!in[x]) continue;
+                const int jj = j[x];
+                Coef a;
+                double su;
+                if (r == 2) {
+                    a = tile_coef_sc(g, jj, i, L.amusc, code[x]);
+                    a.ap = a.ap + sp[x];
+                    su = sp[x] * C.sc_obs + res[x];
+                } else if (r == 0) {
+                    a = tile_coef_u(g, jj, i, L.amu, jj == H - 2, jj == 1, jj == 1 ? g.qy[H - 2][i] : 0.0);
+                    su = mom_source(C, rm, a, ax[x], dp[x], v[x], res[x], C.dpdxm * ax[x] * ay[x], sp[x]);
+                    io.st(S_APU, k[x], a.ap);
+                } else {
+                    a = tile_coef_v(g, jj, i, L.amu, i == W - 2, i == 1, i == 1 ? g.qy[jj][W - 2] : 0.0);
+                    su = mom_source(C, rm, a, ay[x], dp[x], v[x], res[x], C.dpdym * ax[x] * ay[x], sp[x]);
+                    io.st(S_APV, k[x], a.ap);
+                }
+                store_coef(io, e, k[x], a, su);
+                c[x][0] = a.aw; c[x][1] = a.ae; c[x][2] = a.as; c[x][3] = a.an; c[x][4] = a.ap; c[x][5] = su;
+            }
         }
-        cluster_barrier();
+        cluster_arrive();
+    } else if (active) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            if (has[x]) v[x] = io.ld(field, k[x]);
+            if (in[x])
+#pragma unroll
+                for (int a = 0; a < NCOEF; ++a) c[x][a] = io.ld(co_slot(e, a), k[x]);
+        }
     }
-    if (active && mu > 0 && level_smooth_eq<ISOLVE>(L, r == 0 ? EQ_U : r == 1 ? EQ_V : EQ_SC, mu, sm) == 2 &&
-        threadIdx.x == 0)
-        atomicOr(&ST.status, (int)CASE_BAD_LAUNCH);   // the schedule sizes blocks to fit; never taken
-    cluster_barrier();
-    if (active && r == 0) pp_level_body<ISOLVE>(C, ST, L, nu, reduce, fuse, sm);
+    const bool pp = active && r == 0;
+    double d[2][NCOEF];   // CTA 0's p' coefficients
+    auto pp_coefs = [&]() {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            d[x][0] = d[x][1] = d[x][2] = d[x][3] = d[x][5] = 0.0;
+            d[x][4] = 1.0;
+            if (pp && inner[x]) {
+                Coef a;
+                double su;
+                mass_coefp_io(io, C, i, j[x], a, su, S_U, S_V, MC_COEF);
+                d[x][0] = a.aw; d[x][1] = a.ae; d[x][2] = a.as; d[x][3] = a.an; d[x][4] = a.ap;
+            }
+        }
+    };
+    const bool first = EARLY && !what;   // apu and apv are an earlier launch's
+    if (first) pp_coefs();
+    const double *out = phi;
+    if (active) {
+        const double eps = JAC ? 1.0e-30 : 0.0;   // solver's (ap + 1e-30), solvergs' ap
+        const Recip R[2] = {make_recip(JAC ? c[0][4] + eps : c[0][4]), make_recip(JAC ? c[1][4] + eps : c[1][4])};
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (has[x]) {
+                phi[k[x]] = v[x];
+                if (JAC) phi2[k[x]] = v[x];
+            }
+        __syncthreads();
+        out = level_units<ISOLVE>(c, R, in, k, mu, W, phi, phi2);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (in[x]) v[x] = out[k[x]];
+    }
+    cluster_wait();
+    if (active) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            if (in[x] && mu > 0) io.st(field, k[x], v[x]);
+            if (r == 1 && has[x]) st_cluster(&vel[k[x]], 0, v[x]);
+        }
+    }
+    cluster_arrive();
+    // before u and v are there: the p' coefficients, update's other operands
+    if (!first) pp_coefs();
+    double pv[2] = {0.0, 0.0}, divs = 0.0;
+    UpdIn up[2] = {};
+    auto operands = [&](int x) {
+        up[x] = {v[x], 0.0, io.ld(S_P, k[x]), ax[x], ay[x], io.ld(S_APU, k[x]), io.ld(S_APV, k[x]),
+                 (fuse & 4) && L.pcode ? L.pcode[k[x]] : 0};
+    };
+    if (pp) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            if (inner[x]) {
+                if (EARLY) operands(x);
+            } else if (has[x]) {
+                pv[x] = io.ld(S_PP, k[x]);      // boundary ring: masserror leaves it
+            }
+        }
+    }
+    cluster_wait();
+    if (!pp) return;
+    const double eps = JAC ? 1.0e-30 : 0.0;
+    const Recip R[2] = {make_recip(JAC ? d[0][4] + eps : d[0][4]), make_recip(JAC ? d[1][4] + eps : d[1][4])};
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (inner[x]) {
+            Coef a;
+            divs += mass_coefp_io(VisitVel{L, out, vel, ax[x], ay[x]}, C, i, j[x], a, d[x][5], S_U, S_V, MC_SU);
+        }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (has[x]) {
+            phi[k[x]] = pv[x];
+            if (JAC) phi2[k[x]] = pv[x];
+        }
+    __syncthreads();
+    const double *res = level_units<ISOLVE>(d, R, inner, k, nu, W, phi, phi2);
+    const bool outlet = (fuse & 1) && C.ibc_xp == 4;
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (inner[x]) {
+            if (!EARLY) operands(x);
+            up[x].v = vel[k[x]];
+        }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        if (inner[x]) {
+            const int q = k[x];
+            io.st(S_PP, q, res[q]);
+            update_cell(io, C, i, j[x], res[q], res[q + 1], res[q + W], outlet, fuse, up[x]);
+        }
+    if (outlet && t < 2) row_outflow_io(io, t == 0 ? 0 : H - 1, (fuse & 2) != 0);
+    if (reduce) {
+        double a[1] = {divs};
+        block_sum<1>(a);
+        if (t == 0) ST.last_err = a[0];
+    }
+    pp_level_tail(C, C.lv[ig], fuse);
 }
 
 // ------------------------------------------------ band visits (a cluster per case)
@@ -941,19 +1197,6 @@ __device__ __forceinline__ unsigned cl_size_k()
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
     return v;
 }
-// the shared::cluster address `p` (a shared-memory location of this CTA) has in CTA `rank`
-__device__ __forceinline__ unsigned cl_map(const void *p, unsigned rank)
-{
-    unsigned a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-    return a;
-}
-// store v at the shared-memory location `p` has in CTA `rank` of the cluster
-__device__ __forceinline__ void st_cluster(double *p, unsigned rank, double v)
-{
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cl_map(p, rank)), "d"(v) : "memory");
-}
-
 // One CTA's band and this thread's pair: cells (i, ja) and (i, ja + 1).
 struct Band {
     int r, G;
@@ -1735,6 +1978,11 @@ cudaError_t configure_kernels()
                          (const void *)k_smooth_tma<MGFVM_GAUSS_SEIDEL, SMOOTH_BLOCK / 4>};
     for (const void *f : tma)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMOOTH_TMA_SMEM_MAX);
+    const void *visit[] = {(const void *)k_level_visit<MGFVM_JACOBI, VISIT_BLOCK>, (const void *)k_level_visit<MGFVM_JACOBI, SMOOTH_BLOCK>,
+                           (const void *)k_level_visit<MGFVM_GAUSS_SEIDEL, VISIT_BLOCK>,
+                           (const void *)k_level_visit<MGFVM_GAUSS_SEIDEL, SMOOTH_BLOCK>};
+    for (const void *f : visit)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, VISIT_SMEM_MAX);
     const void *band[] = {(const void *)k_band_visit<MGFVM_JACOBI>, (const void *)k_band_visit<MGFVM_GAUSS_SEIDEL>};
     for (const void *f : band)
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, BAND_SMEM_MAX);
@@ -1871,9 +2119,12 @@ cudaError_t launch_one(const Launch &X, const CaseDev *dc, CaseState *ds, const 
     case K_LEVEL_VISIT:
         if (b > SMOOTH_BLOCK || g.x != 3) return cudaErrorInvalidValue;
         if (S.isolve == MGFVM_JACOBI)
-            le = launch_k(pdl, k_level_visit<MGFVM_JACOBI>, g, b, X.smem, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2, X.a3, X.a4);
+            le = launch_k(pdl, b <= VISIT_BLOCK ? k_level_visit<MGFVM_JACOBI, VISIT_BLOCK> : k_level_visit<MGFVM_JACOBI, SMOOTH_BLOCK>,
+                          g, b, X.smem, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2, X.a3, X.a4);
         else
-            le = launch_k(pdl, k_level_visit<MGFVM_GAUSS_SEIDEL>, g, b, X.smem, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2, X.a3, X.a4);
+            le = launch_k(pdl, b <= VISIT_BLOCK ? k_level_visit<MGFVM_GAUSS_SEIDEL, VISIT_BLOCK>
+                                                : k_level_visit<MGFVM_GAUSS_SEIDEL, SMOOTH_BLOCK>,
+                          g, b, X.smem, st, dc, ds, X.ig, X.mode, X.a0, X.a1, X.a2, X.a3, X.a4);
         break;
     case K_COARSE_CYCLE:
         if (b > SMOOTH_BLOCK || g.x != 3) return cudaErrorInvalidValue;

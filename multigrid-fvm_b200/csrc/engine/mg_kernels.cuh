@@ -77,6 +77,10 @@ struct Sched {
 // SM) threads, one vertical cell pair per thread, covers a tile plus a halo of one cell
 // per unit on every side.
 constexpr int SMOOTH_BLOCK = 1024;
+// one-CTA level visits: blocks up to this size leave a thread 96 registers; and the field (a
+// second buffer for Jacobi), v and four arrays for the assembly, of at most 2 SMOOTH_BLOCK cells
+constexpr int VISIT_BLOCK = 640;
+constexpr int VISIT_SMEM_MAX = 7 * 2 * SMOOTH_BLOCK * (int)sizeof(double);
 // band visits: at most 8 CTAs per case (the portable cluster size) and this much
 // dynamic shared memory per CTA (the band and its two halo rows, two buffers for Jacobi)
 constexpr int BAND_MAX_CTAS = 8;
