@@ -476,14 +476,21 @@ __device__ __forceinline__ double gs_value_r(double aw, double ae, double as, do
     return div_by(nb + su, R);
 }
 
-// jacobi_value with R = make_recip(ap + 1.0e-30)
+// jacobi_value with R = make_recip(ap + 1.0e-30).  A quotient that markstein gives is neither
+// zero nor infinite, so with a finite pc the weighted sum 0 pc + 1 g is g: two operations less
+// of the FP64 pipe, which bounds a sweep.
+static __device__ __noinline__ double jacobi_rare(double a, double b, double y, double pc)
+{
+    const double wj = 1.0;
+    const double g = div_by_rare(a, b, y);
+    return (1.0 - wj) * pc + wj * g;
+}
 __device__ __forceinline__ double jacobi_value_r(double aw, double ae, double as, double an, const Recip &R,
                                                  double su, double pw, double pe, double ps, double pn, double pc)
 {
-    const double wj = 1.0;
-    double nb = aw * pw + ae * pe + as * ps + an * pn;
-    double g = div_by(nb + su, R);
-    return (1.0 - wj) * pc + wj * g;
+    const double nb = aw * pw + ae * pe + as * ps + an * pn, a = nb + su;
+    if (div_plain(a, R) & ((__double2hiint(pc) & 0x7ff00000) != 0x7ff00000)) return markstein(a, R);
+    return jacobi_rare(a, R.b, R.y, pc);
 }
 
 template <class IO>

@@ -408,7 +408,8 @@ struct PairTile {
 
 // 0: this CTA has work, 1: it has none, 2: the launch is too small for its region.
 // `bx` picks the tile (blockIdx.x in the tiled smoothers) of the domain, whose rows are npx
-// cells apart.
+// cells apart.  COLOURS: cell A is the pair's red one, B its black one; else A is the lower.
+template <bool COLOURS = true>
 __device__ __forceinline__ int pair_tile(const Dom &dom, int npx, int nu, int tile, PairTile &P, int bx)
 {
     P.d = dom;
@@ -436,7 +437,7 @@ __device__ __forceinline__ int pair_tile(const Dom &dom, int npx, int nu, int ti
     const int i = P.rx0 + c, jr = P.ry0 + r;
     const bool two = own && r + 1 < P.Hh;
     P.i = i;
-    P.jA = ((i + jr) & 1) == 0 ? jr : jr + 1;
+    P.jA = !COLOURS || ((i + jr) & 1) == 0 ? jr : jr + 1;
     P.jB = P.jA == jr ? jr + 1 : jr;
     P.okA = own && (P.jA == jr || two);
     P.okB = own && (P.jB == jr || two);
@@ -459,6 +460,58 @@ __device__ __forceinline__ int pair_tile(const LevelDev &L, int e, int nu, int t
     return pair_tile(dom_eq(L, e), L.npx, nu, tile, P, bx);
 }
 
+// Units u0 .. u0 + n - 1 of a region in shared memory (phi; Jacobi's second buffer phi2; rows
+// of W) by vertical pairs: a thread's cells 0 and 1, at kA and kB with values v, coefficients c
+// and reciprocals R, are in unit h's window while h <= limA, limB.  Gauss-Seidel: cell 0 is
+// red, cell 1 black; Jacobi: cell 0 is the lower.  Barriers before and after.
+// Bound by shared memory (8 bytes a lane, two wavefronts an access): the pair's other cell and
+// the cell itself come from registers, so a half-sweep reads three values and writes one (from
+// four and one), a sweep of two cells reads six and writes two (from ten and two).  V-cycles
+// of a 64^2 channel (Jacobi) 86 us against 94, of three 304 x 112 ducts (Jacobi) 177 against
+// 200, of two 256^2 cases (Gauss-Seidel) 238 against 244.
+template <int ISOLVE>
+__device__ __forceinline__ void pair_units(const double (&c)[2][NCOEF], const Recip (&R)[2], double (&v)[2], int limA,
+                                           int limB, int kA, int kB, int u0, int n, int W, double *phi, double *phi2)
+{
+    if (ISOLVE == MGFVM_JACOBI) {
+        for (int h = 1; h <= n; ++h) {
+            const double *cur = ((h - 1) & 1) ? phi2 : phi;
+            double *nxt = ((h - 1) & 1) ? phi : phi2;
+            const double a = v[0], b = v[1];
+            if (h <= limA) {
+                v[0] = jacobi_value_r(c[0][0], c[0][1], c[0][2], c[0][3], R[0], c[0][5], cur[kA - 1], cur[kA + 1], cur[kA - W],
+                                      b, a);
+                nxt[kA] = v[0];
+            }
+            if (h <= limB) {
+                v[1] = jacobi_value_r(c[1][0], c[1][1], c[1][2], c[1][3], R[1], c[1][5], cur[kB - 1], cur[kB + 1], a,
+                                      cur[kB + W], b);
+                nxt[kB] = v[1];
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const bool up = kA < kB;   // the black cell is the red one's northern neighbour
+    const int far = up ? -W : W;
+    for (int h = 1; h <= n; ++h) {
+        if (((u0 + h - 1) & 1) == 0) {
+            if (h <= limA) {
+                const double o = phi[kA + far];
+                v[0] = gs_value_r(c[0][0], c[0][1], c[0][2], c[0][3], R[0], c[0][5], phi[kA - 1], phi[kA + 1], up ? o : v[1],
+                                  up ? v[1] : o);
+                phi[kA] = v[0];
+            }
+        } else if (h <= limB) {
+            const double o = phi[kB - far];
+            v[1] = gs_value_r(c[1][0], c[1][1], c[1][2], c[1][3], R[1], c[1][5], phi[kB - 1], phi[kB + 1], up ? v[0] : o,
+                              up ? o : v[0]);
+            phi[kB] = v[1];
+        }
+        __syncthreads();
+    }
+}
+
 // Temporal-blocked smoother.  blockIdx.z picks an equation of `mask`, blockIdx.x a
 // tile.  The CTA stages its region: every thread owns one vertical pair of cells,
 // holds both cells' six coefficients in registers and their field values in shared
@@ -476,93 +529,62 @@ template <int ISOLVE, int NT, bool EARLY>
 __global__ void __launch_bounds__(NT, SMOOTH_BLOCK / NT) k_smooth(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int mask, int u0, int nu,
                                                          int dir, int tile)
 {
-    if (!EARLY) pdl_enter();
+    constexpr bool JAC = ISOLVE == MGFVM_JACOBI;
     extern __shared__ double sm[];
     const CaseDev &C = cs[blockIdx.y];
-    if (!case_active(C, st[blockIdx.y], ig, mode)) return;
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
     const int e = nth_eq(mask, blockIdx.z);
-    const LevelDev &L = C.lv[ig];
     PairTile P;
-    const int g = pair_tile(L, e, nu, tile, P, blockIdx.x);
+    const int g = mode_active(C, ig, mode)
+                      ? pair_tile<!JAC>(Dom{1, 1, L.npx - (e == EQ_U ? 3 : 2), L.npy - (e == EQ_V ? 3 : 2)}, L.npx, nu, tile, P, blockIdx.x)
+                      : 1;
+    double c[2][NCOEF], v[2] = {0.0, 0.0};
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        c[x][0] = c[x][1] = c[x][2] = c[x][3] = c[x][5] = 0.0;
+        c[x][4] = 1.0;
+    }
+    auto coefs = [&]() {
+#pragma unroll
+        for (int a = 0; a < NCOEF; ++a) {
+            const double *k = io.at(co_slot(e, a));
+            if (P.limA >= 0) c[0][a] = k[P.gA];
+            if (P.limB >= 0) c[1][a] = k[P.gB];
+        }
+    };
+    if (EARLY && g == 0) coefs();
+    pdl_enter();
     if (g == 1) return;
+    const bool live = !st[blockIdx.y].done;
     if (g == 2) {     // the schedule sizes blocks to fit; never taken
-        if (threadIdx.x == 0) atomicOr(&st[blockIdx.y].status, (int)CASE_BAD_LAUNCH);
+        if (live && threadIdx.x == 0) atomicOr(&st[blockIdx.y].status, (int)CASE_BAD_LAUNCH);
         return;
     }
-    const int W = P.W, kA = P.kA, kB = P.kB, limA = P.limA, limB = P.limB;
-    const int fs = eq_field(e), ts = eq_tmp(e);
-    const double *src = L.f[dir == 1 ? ts : fs];
-    double *dst = L.f[dir == 0 ? ts : fs];
-    double *phi = sm, *phi2 = sm + W * P.Hh;
-    const double *__restrict__ gaw = L.f[co_slot(e, CK_AW)];
-    const double *__restrict__ gae = L.f[co_slot(e, CK_AE)];
-    const double *__restrict__ gas = L.f[co_slot(e, CK_AS)];
-    const double *__restrict__ gan = L.f[co_slot(e, CK_AN)];
-    const double *__restrict__ gap = L.f[co_slot(e, CK_AP)];
-    const double *__restrict__ gsu = L.f[co_slot(e, CK_SU)];
-    double A[6] = {0, 0, 0, 0, 0, 0}, B[6] = {0, 0, 0, 0, 0, 0}, pA = 0.0, pB = 0.0;
-    if (EARLY) {
-        if (P.okA) {
-            const int g0 = P.gA;
-            A[0] = gaw[g0]; A[1] = gae[g0]; A[2] = gas[g0]; A[3] = gan[g0]; A[4] = gap[g0]; A[5] = gsu[g0];
-        }
-        if (P.okB) {
-            const int g0 = P.gB;
-            B[0] = gaw[g0]; B[1] = gae[g0]; B[2] = gas[g0]; B[3] = gan[g0]; B[4] = gap[g0]; B[5] = gsu[g0];
-        }
-        pdl_enter();
-        if (P.okA) pA = src[P.gA];
-        if (P.okB) pB = src[P.gB];
-    } else {
-        if (P.okA) {
-            const int g0 = P.gA;
-            pA = src[g0];
-            A[0] = gaw[g0]; A[1] = gae[g0]; A[2] = gas[g0]; A[3] = gan[g0]; A[4] = gap[g0]; A[5] = gsu[g0];
-        }
-        if (P.okB) {
-            const int g0 = P.gB;
-            pB = src[g0];
-            B[0] = gaw[g0]; B[1] = gae[g0]; B[2] = gas[g0]; B[3] = gan[g0]; B[4] = gap[g0]; B[5] = gsu[g0];
-        }
+    {
+        const double *src = io.at(dir == 1 ? eq_tmp(e) : eq_field(e));
+        if (P.okA) v[0] = src[P.gA];
+        if (P.okB) v[1] = src[P.gB];
     }
-    const double eps = ISOLVE == MGFVM_JACOBI ? 1.0e-30 : 0.0;   // solver's (ap + 1e-30), solvergs' ap
-    const Recip RA = make_recip(ISOLVE == MGFVM_JACOBI ? A[4] + eps : A[4]);
-    const Recip RB = make_recip(ISOLVE == MGFVM_JACOBI ? B[4] + eps : B[4]);
+    if (!EARLY) coefs();
+    if (!live) return;
+    const int W = P.W, kA = P.kA, kB = P.kB;
+    double *phi = sm, *phi2 = sm + W * P.Hh;
+    const double eps = JAC ? 1.0e-30 : 0.0;   // solver's (ap + 1e-30), solvergs' ap
+    const Recip R[2] = {make_recip(JAC ? c[0][4] + eps : c[0][4]), make_recip(JAC ? c[1][4] + eps : c[1][4])};
     if (P.okA) {
-        phi[kA] = pA;
-        if (ISOLVE == MGFVM_JACOBI) phi2[kA] = pA;
+        phi[kA] = v[0];
+        if (JAC) phi2[kA] = v[0];
     }
     if (P.okB) {
-        phi[kB] = pB;
-        if (ISOLVE == MGFVM_JACOBI) phi2[kB] = pB;
+        phi[kB] = v[1];
+        if (JAC) phi2[kB] = v[1];
     }
     __syncthreads();
-    for (int h = 1; h <= nu; ++h) {
-        if (ISOLVE == MGFVM_GAUSS_SEIDEL) {
-            if (((u0 + h - 1) & 1) == 0) {
-                if (h <= limA)
-                    phi[kA] = gs_value_r(A[0], A[1], A[2], A[3], RA, A[5], phi[kA - 1], phi[kA + 1], phi[kA - W],
-                                         phi[kA + W]);
-            } else {
-                if (h <= limB)
-                    phi[kB] = gs_value_r(B[0], B[1], B[2], B[3], RB, B[5], phi[kB - 1], phi[kB + 1], phi[kB - W],
-                                         phi[kB + W]);
-            }
-        } else {
-            const double *cur = ((h - 1) & 1) ? phi2 : phi;
-            double *nxt = ((h - 1) & 1) ? phi : phi2;
-            if (h <= limA)
-                nxt[kA] = jacobi_value_r(A[0], A[1], A[2], A[3], RA, A[5], cur[kA - 1], cur[kA + 1], cur[kA - W],
-                                         cur[kA + W], cur[kA]);
-            if (h <= limB)
-                nxt[kB] = jacobi_value_r(B[0], B[1], B[2], B[3], RB, B[5], cur[kB - 1], cur[kB + 1], cur[kB - W],
-                                         cur[kB + W], cur[kB]);
-        }
-        __syncthreads();
-    }
-    const double *res = (ISOLVE == MGFVM_JACOBI && (nu & 1)) ? phi2 : phi;
-    if (P.outA) dst[P.gA] = res[kA];
-    if (P.outB) dst[P.gB] = res[kB];
+    pair_units<ISOLVE>(c, R, v, P.limA, P.limB, kA, kB, u0, nu, W, phi, phi2);
+    double *dst = io.at(dir == 0 ? eq_tmp(e) : eq_field(e));
+    if (P.outA) dst[P.gA] = v[0];
+    if (P.outB) dst[P.gB] = v[1];
 }
 
 // ------------------------------------------------ TMA-staged tile smoother
@@ -904,34 +926,6 @@ struct LevelGeo {
     Rows cx, cy, qx, qy;
 };
 
-// The units 1 .. n of a level in shared memory (phi; Jacobi's second buffer phi2): a thread's
-// red cell 0 and black cell 1 at k with coefficients c, reciprocals R, in the domain where
-// `in`.  Barriers before and after.  Returns the buffer that holds the result.
-template <int ISOLVE>
-__device__ __forceinline__ const double *level_units(const double (&c)[2][NCOEF], const Recip (&R)[2], const bool (&in)[2],
-                                                     const int (&k)[2], int n, int W, double *phi, double *phi2)
-{
-    for (int h = 1; h <= n; ++h) {
-        const double *cur = ISOLVE == MGFVM_JACOBI && ((h - 1) & 1) ? phi2 : phi;
-        double *nxt = ISOLVE == MGFVM_JACOBI && ((h - 1) & 1) ? phi : ISOLVE == MGFVM_JACOBI ? phi2 : phi;
-        if (ISOLVE == MGFVM_JACOBI) {
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-                if (in[x]) {
-                    const int q = k[x];
-                    nxt[q] = jacobi_value_r(c[x][0], c[x][1], c[x][2], c[x][3], R[x], c[x][5], cur[q - 1], cur[q + 1],
-                                            cur[q - W], cur[q + W], cur[q]);
-                }
-        } else if ((h & 1) ? in[0] : in[1]) {
-            const int q = (h & 1) ? k[0] : k[1];
-            const double(&a)[NCOEF] = (h & 1) ? c[0] : c[1];
-            nxt[q] = gs_value_r(a[0], a[1], a[2], a[3], (h & 1) ? R[0] : R[1], a[5], cur[q - 1], cur[q + 1], cur[q - W], cur[q + W]);
-        }
-        __syncthreads();
-    }
-    return ISOLVE == MGFVM_JACOBI && (n & 1) ? phi2 : phi;
-}
-
 // u, v of a visit's p' sources: from shared memory, with the cell's own face areas.
 struct VisitVel {
     using T = double;
@@ -973,7 +967,8 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
     const int W = L.npx, H = L.npy, n = W * H, r = blockIdx.x, t = threadIdx.x;
     const int e = r == 0 ? EQ_U : r == 1 ? EQ_V : EQ_SC, field = eq_field(e);
     const int i = t % W, j0 = 2 * (t / W);
-    const int j[2] = {((i + j0) & 1) == 0 ? j0 : j0 + 1, ((i + j0) & 1) == 0 ? j0 + 1 : j0};
+    const bool red = JAC || ((i + j0) & 1) == 0;   // the lower cell is cell 0
+    const int j[2] = {red ? j0 : j0 + 1, red ? j0 + 1 : j0};
     const int k[2] = {j[0] * W + i, j[1] * W + i};
     bool has[2], inner[2], in[2];   // a cell of the padded level, of its interior, of the equation's domain
     double ax[2] = {0.0, 0.0}, ay[2] = {0.0, 0.0}, sp[2] = {0.0, 0.0};
@@ -1084,7 +1079,6 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
     };
     const bool first = EARLY && !what;   // apu and apv are an earlier launch's
     if (first) pp_coefs();
-    const double *out = phi;
     if (active) {
         const double eps = JAC ? 1.0e-30 : 0.0;   // solver's (ap + 1e-30), solvergs' ap
         const Recip R[2] = {make_recip(JAC ? c[0][4] + eps : c[0][4]), make_recip(JAC ? c[1][4] + eps : c[1][4])};
@@ -1095,11 +1089,9 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
                 if (JAC) phi2[k[x]] = v[x];
             }
         __syncthreads();
-        out = level_units<ISOLVE>(c, R, in, k, mu, W, phi, phi2);
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-            if (in[x]) v[x] = out[k[x]];
+        pair_units<ISOLVE>(c, R, v, in[0] ? mu : 0, in[1] ? mu : 0, k[0], k[1], 0, mu, W, phi, phi2);
     }
+    const double *out = JAC && (mu & 1) ? phi2 : phi;
     cluster_wait();
     if (active) {
 #pragma unroll
@@ -1145,7 +1137,8 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
             if (JAC) phi2[k[x]] = pv[x];
         }
     __syncthreads();
-    const double *res = level_units<ISOLVE>(d, R, inner, k, nu, W, phi, phi2);
+    pair_units<ISOLVE>(d, R, pv, inner[0] ? nu : 0, inner[1] ? nu : 0, k[0], k[1], 0, nu, W, phi, phi2);
+    const double *res = JAC && (nu & 1) ? phi2 : phi;
     const bool outlet = (fuse & 1) && C.ibc_xp == 4;
 #pragma unroll
     for (int x = 0; x < 2; ++x)
@@ -2186,7 +2179,7 @@ __global__ void __launch_bounds__(SMOOTH_BLOCK, 1)
 {
     extern __shared__ double sm[];
     PairTile P;
-    if (pair_tile(Dom{1, 1, wi, wj}, npx, nu, tile, P, blockIdx.x) != 0) {
+    if (pair_tile<false>(Dom{1, 1, wi, wj}, npx, nu, tile, P, blockIdx.x) != 0) {
         pdl_enter();
         return;   // (the launch is sized to its tiles)
     }
@@ -2212,19 +2205,7 @@ __global__ void __launch_bounds__(SMOOTH_BLOCK, 1)
     for (int x = 0; x < 2; ++x)
         if (ok[x]) phi[k2[x]] = phi2[k2[x]] = v[x];
     __syncthreads();
-    for (int h = 1; h <= nu; ++h) {
-        const double *cur = ((h - 1) & 1) ? phi2 : phi;
-        double *nxt = ((h - 1) & 1) ? phi : phi2;
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-            if (h <= lim[x]) {
-                const int k = k2[x];
-                v[x] = jacobi_value_r(c[x][0], c[x][1], c[x][2], c[x][3], R[x], c[x][5], cur[k - 1], cur[k + 1],
-                                      cur[k - W], cur[k + W], cur[k]);
-                nxt[k] = v[x];
-            }
-        __syncthreads();
-    }
+    pair_units<MGFVM_JACOBI>(c, R, v, lim[0], lim[1], k2[0], k2[1], 0, nu, W, phi, phi2);
 #pragma unroll
     for (int x = 0; x < 2; ++x)
         if (out[x]) dst[g2[x]] = v[x];
