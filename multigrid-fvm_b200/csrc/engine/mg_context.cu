@@ -398,6 +398,41 @@ struct Builder {
         }
         return t_best < t_old;
     }
+    // Mixed precision's plan (k_smooth_q32), any number of launches; false where the tuning asks
+    // for k_smooth_f32's.  Its times, 4 us a round of CTAs (two an SM) and 0.2 a unit, choose
+    // the fastest of one to six launches on 1, 12 and 24 cases of 256^2 and one of 1024^2 (p'
+    // of 12 cases: 18.3 us a launch of seven units, 27 of ten; V-cycle 0.474 against 0.478 ms).
+    bool smooth_q32_plan(int ig, int neq, int units, QPlan &best) const
+    {
+        if (x->sched.isolve != MGFVM_GAUSS_SEIDEL || x->tune.smooth_threads[ig] || x->tune.smooth_units[ig]) return false;
+        int wi = 0, wj = 0;
+        for (const mgfvm_config &c : x->cfg)
+            if (ig < c.ngrid) {
+                if (npx_of(c, ig) & 1) return false;   // (never: rows are loaded in pairs)
+                wi = std::max(wi, npx_of(c, ig) - 2);
+                wj = std::max(wj, npy_of(c, ig) - 2);
+            }
+        auto side = [](int n, int most) { return (n + (n + most - 1) / most - 1) / ((n + most - 1) / most); };
+        double t_best = 1e300;
+        for (int c = 1; c <= units; ++c) {
+            const int u = (units + c - 1) / c, mx = SMOOTH_Q_COLS - 2 * u - 1, my = SMOOTH_Q_ROWS - 2 * u - 1;
+            if (mx < MIN_TILE || my < MIN_TILE) continue;
+            QPlan p{c, side(wi, mx), side(wj, my), 1};
+            long long n = 0;
+            for (const mgfvm_config &g : x->cfg)
+                if (ig < g.ngrid) {
+                    const int t = ((npx_of(g, ig) - 2 + p.tw - 1) / p.tw) * ((npy_of(g, ig) - 2 + p.th - 1) / p.th);
+                    p.tiles = std::max(p.tiles, t);
+                    n += (long long)t * neq;
+                }
+            const double t = c * (0.5 + (double)((n + 2 * SMS - 1) / (2 * SMS)) * (4.0 + 0.2 * u));
+            if (t < t_best) {
+                t_best = t;
+                best = p;
+            }
+        }
+        return t_best < 1e300;
+    }
     int f32_buf = 0;   // the FP32 correction buffer the last F32 smoothing call ended in
     bool smooth(int ig, int mode, int mask, int nsw, bool tmp_ok = false)
     {
@@ -408,6 +443,23 @@ struct Builder {
         const int bufs = isolve == MGFVM_JACOBI ? 2 : 1;
         const int kern = K_SMOOTH;
         auto smem_for = [&](int cells) { return bufs * cells * (int)sizeof(double); };
+        QPlan qp;
+        if (f32_level(ig, mode) && smooth_q32_plan(ig, neq, units, qp)) {
+            int u0 = 0;
+            for (int c = 0; c < qp.chunks; ++c) {
+                const int nu = units / qp.chunks + (c < units % qp.chunks ? 1 : 0);
+                const int flags = (c == 0 ? 1 : 0) | (c == qp.chunks - 1 ? 2 : 0) | ((c & 1) ? 4 : 0) |
+                                  (c > 0 && x->sched.pdl ? 8 : 0);   // as below
+                Launch &L = add(K_SMOOTH_F32, ig, mode, 0, mask, u0, nu, flags);
+                L.bw = qp.tw;
+                L.bh = qp.th;
+                L.grid = dim3((unsigned)qp.tiles, x->ncases, neq);
+                L.block = SMOOTH_Q_THREADS;
+                u0 += nu;
+            }
+            f32_buf = qp.chunks & 1;
+            return false;
+        }
         if (f32_level(ig, mode)) {
             // launches of at most the level's cap of units; the correction passes between
             // them in FP32 and the last adds it to the field, so any count works
@@ -444,7 +496,6 @@ struct Builder {
             L.smem = smem_for(mx * my);
             return false;
         }
-        QPlan qp;
         if (smooth_q_plan(ig, neq, units, tmp_ok, qp)) {
             int u0 = 0;
             // more tiles than SMs: CTAs that go through a table of them

@@ -2086,6 +2086,10 @@ cudaError_t launch_one(const Launch &X, const CaseDev *dc, CaseState *ds, const 
             le = launch_smooth<MGFVM_GAUSS_SEIDEL>(pdl, X, g, b, dc, ds, st);
         break;
     case K_SMOOTH_F32:
+        if (X.bw) {
+            le = launch_smooth_q32(X, dc, ds, S, st);
+            break;
+        }
         if (b > SMOOTH_BLOCK) return cudaErrorInvalidValue;
         if (S.isolve == MGFVM_JACOBI) {
             if (X.a3 & 8) le = launch_smooth_f32<MGFVM_JACOBI, true>(pdl, X, g, b, dc, ds, st);

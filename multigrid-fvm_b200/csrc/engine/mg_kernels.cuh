@@ -49,7 +49,7 @@ struct Launch {
     dim3 grid;
     int block;
     int smem;
-    int bw, bh;        // K_SMOOTH_TMA: box width and height; K_SMOOTH_Q: tile
+    int bw, bh;        // K_SMOOTH_TMA: box width and height; K_SMOOTH_Q, K_SMOOTH_F32: tile (0: a4)
     int box;           // K_SMOOTH_Q by a table of a4 tiles: box width << 16 | height
     int map;           // these: index of its first tensor-map pair in the schedule's table
     int tile0;         // K_SMOOTH_Q by a table: index of its first tile in the schedule's
@@ -122,6 +122,7 @@ struct alignas(16) QTile {
     int npx, npy, tx, ty, icase, e;
 };
 cudaError_t configure_smooth_q();
+cudaError_t launch_smooth_q32(const Launch &L, const CaseDev *dcases, CaseState *dstate, const Sched &S, cudaStream_t stream);
 // The same on a caller's own level (mgfvm_rbgs_f64): the expected time of its plan, and the
 // launches (`tmp` unused where chunks is 1).
 double raw_q_plan(int wi, int wj, int units, int &chunks, int &tw, int &th);

@@ -394,6 +394,139 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1) r_smooth_q(QIn in, int u0
     });
 }
 
+// Mixed precision: the same blocks, regions and units on the FP32 operands and corrections of
+// k_smooth_f32 (mg_kernels.cu), with its `flags` and its bits; a division less, so no
+// reciprocals, and half the registers: two CTAs an SM, one's loads under the other's units.
+// A thread's eight cells take their operands in 28 paired loads where k_smooth_f32's pair a
+// thread had 2048 cells an SM, most of them halo at ten units.  Bound by the operands' way
+// from memory (4 us a round of CTAs).  Level 0 of 12 256^2 cases: u, v, sc and p' 95 us in four
+// launches against 206 in three; a V-cycle 0.474 ms against 0.654, of one 1024^2 case 0.646.
+template <bool EARLY>
+__global__ void __launch_bounds__(SMOOTH_Q_THREADS, 2)
+    k_smooth_q32(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int mask, int u0, int nu, int flags,
+                 int tw, int th)
+{
+    __shared__ float smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
+    float *del = smq + 2 * QX;   // a row of slack on either side
+    const CaseDev &C = cs[blockIdx.y];
+    const FastLevel L = fast_level(C.lv[ig]);
+    const Fast io{L};
+    const int e = nth_eq(mask, blockIdx.z), npx = L.npx, t = threadIdx.x, qx = t % QX, qy = t / QX;
+    const int dx1 = npx - (e == EQ_U ? 3 : 2), dy1 = L.npy - (e == EQ_V ? 3 : 2);
+    const int txn = max(1, (dx1 + tw - 1) / tw), tx = blockIdx.x % txn, ty = blockIdx.x / txn;
+    const bool active = mode_active(C, ig, mode) && dx1 >= 1 && dy1 >= 1 && ty * th < dy1;
+    const bool first = (flags & 1) != 0, last = (flags & 2) != 0;
+    const QTileAt T = tile_at(dx1, dy1, tx, ty, tw, th, nu, qx, qy);
+    const int i = T.i, j = T.j, q0 = j * npx + i;
+    auto buf = [&](int b) { return reinterpret_cast<float *>(io.at(eq_tmp(e))) + (b ? (size_t)npx * L.npy : 0); };
+    // cell (x, y) of the block: aw, ae, as, an, 1 / ap, r; v the correction
+    float w[BY][BX], ea[BY][BX], so[BY][BX], no[BY][BX], ra[BY][BX], rs[BY][BX], v[BY][BX];
+    auto load = [&](const float *p, float (&a)[BY][BX]) {
+#pragma unroll
+        for (int y = 0; y < BY; ++y) {
+            a[y][0] = a[y][1] = 0.0f;
+            if (active && T.mine && j + y <= T.ry1) {
+                // (a level that has a coarser one has an even number of cells a row)
+                const float2 d = *reinterpret_cast<const float2 *>(p + q0 + y * npx);
+                a[y][0] = d.x;
+                a[y][1] = d.y;
+            }
+        }
+    };
+    auto op = [&](int k) { return reinterpret_cast<const float *>(io.at(co_slot(e, k))); };
+    auto operands = [&]() {
+        load(op(CK_AW), w);
+        load(op(CK_AE), ea);
+        load(op(CK_AS), so);
+        load(op(CK_AN), no);
+        load(op(CK_AP), ra);
+        load(op(CK_SU), rs);
+    };
+    if (EARLY) operands();
+    pdl_enter();
+    if (!active) return;
+    const bool live = !st[blockIdx.y].done;
+    if (!EARLY) operands();
+    if (first) {
+#pragma unroll
+        for (int y = 0; y < BY; ++y) v[y][0] = v[y][1] = 0.0f;
+    } else {
+        load(buf((flags & 4) ? 1 : 0), v);
+    }
+    if (!live) return;
+    if (qy < QY) {
+#pragma unroll
+        for (int y = 0; y < BY; ++y)
+#pragma unroll
+            for (int x = 0; x < BX; ++x) del[sh(BY * qy + y, x, qx)] = v[y][x];
+    }
+    __syncthreads();
+    for (int h = 1; h <= nu; ++h) {
+        const int g = nu - h;
+        const int xl = max(1, T.x0 - g), xr = min(dx1, T.x1 + g), yl = max(1, T.y0 - g), yr = min(dy1, T.y1 + g);
+        bool ax[BX], ay[BY];
+#pragma unroll
+        for (int x = 0; x < BX; ++x) ax[x] = i + x >= xl && i + x <= xr;
+#pragma unroll
+        for (int y = 0; y < BY; ++y) ay[y] = j + y >= yl && j + y <= yr;
+        auto unit = [&](auto tag) {
+            constexpr int COL = decltype(tag)::value;
+            if (qy >= QY) return;
+            float z[BY];
+#pragma unroll
+            for (int y = 0; y < BY; ++y) {
+                const int x = (y + COL) & 1, r = BY * qy + y;
+                const float pw = x == 0 ? del[sh(r, 1, qx - 1)] : v[y][0];
+                const float pe = x == 1 ? del[sh(r, 0, qx + 1)] : v[y][1];
+                const float ps = y == 0 ? del[sh(r - 1, x, qx)] : v[y - 1][x];
+                const float pn = y == BY - 1 ? del[sh(r + 1, x, qx)] : v[y + 1][x];
+                z[y] = (w[y][x] * pw + ea[y][x] * pe + so[y][x] * ps + no[y][x] * pn + rs[y][x]) * ra[y][x];
+            }
+#pragma unroll
+            for (int y = 0; y < BY; ++y) {
+                const int x = (y + COL) & 1;
+                if (ax[x] && ay[y]) {
+                    v[y][x] = z[y];
+                    del[sh(BY * qy + y, x, qx)] = z[y];
+                }
+            }
+        };
+        if (((u0 + h - 1) & 1) == 0) unit(std::integral_constant<int, 0>{});
+        else unit(std::integral_constant<int, 1>{});
+        __syncthreads();
+    }
+    // the tile, and zero on the boundary ring where it touches it
+    const int ox0 = T.x0 == 1 ? 0 : T.x0, ox1 = T.x1 == dx1 ? dx1 + 1 : T.x1;
+    const int oy0 = T.y0 == 1 ? 0 : T.y0, oy1 = T.y1 == dy1 ? dy1 + 1 : T.y1;
+    float *dst = buf((flags & 4) ? 0 : 1);
+    double *phi = io.at(eq_field(e));
+    const bool add = last && e != EQ_PP;
+    if (T.mine) {
+        auto out = [&](int x, int y) { return i + x >= ox0 && i + x <= ox1 && j + y >= oy0 && j + y <= oy1; };
+        auto dom = [&](int x, int y) { return i + x >= 1 && i + x <= dx1 && j + y >= 1 && j + y <= dy1; };
+        double f[BY][BX];   // (all read before the first is written: the loads stay together)
+#pragma unroll
+        for (int y = 0; y < BY; ++y)
+#pragma unroll
+            for (int x = 0; x < BX; ++x) f[y][x] = add && out(x, y) && dom(x, y) ? phi[q0 + y * npx + x] : 0.0;
+#pragma unroll
+        for (int y = 0; y < BY; ++y)
+#pragma unroll
+            for (int x = 0; x < BX; ++x)
+                if (out(x, y)) {
+                    const int q = q0 + y * npx + x;
+                    dst[q] = dom(x, y) ? v[y][x] : 0.0f;
+                    if (add && dom(x, y)) phi[q] = f[y][x] + (double)v[y][x];
+                }
+    }
+}
+
+cudaError_t launch_smooth_q32(const Launch &X, const CaseDev *dc, CaseState *ds, const Sched &S, cudaStream_t st)
+{
+    return launch_k(S.pdl, (X.a3 & 8) ? k_smooth_q32<true> : k_smooth_q32<false>, X.grid, SMOOTH_Q_THREADS, 0, st, dc, ds,
+                    X.ig, X.mode, X.a0, X.a1, X.a2, X.a3 & 7, X.bw, X.bh);
+}
+
 cudaError_t configure_smooth_q()
 {
     cudaError_t e = cudaSuccess;
