@@ -130,7 +130,7 @@ def smoother_roofline(solver, cases, traffic=None, reps=20):
     achieved = algo_bytes / (per_launch_ms / 1e3) / 1e9
     return {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": traffic,
-            "kernel": "k_smooth (shared-memory tile smoother, p' equation, level 0)",
+            "kernel": "Gauss-Seidel tile smoother (k_smooth_q; k_smooth under a tuned schedule), p' equation, level 0",
             "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
             "per_launch_us": round(per_launch_ms * 1e3, 3), "launches_per_op": klaunch // reps,
             "algorithmic_bytes_per_launch": int(algo_bytes)}
