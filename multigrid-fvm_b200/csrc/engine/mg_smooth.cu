@@ -111,6 +111,7 @@ __device__ __forceinline__ void prepare_block(QBlock &B, const QTileAt &T, int d
 }
 // The units u0 .. u0 + nu - 1 (each between barriers; one precedes the first), then the tile,
 // plus the boundary ring where it touches it, to dst.
+template <bool MEND>
 __device__ __forceinline__ void smooth_block(QBlock &B, const QTileAt &T, int dx1, int dy1, int npx, double *phi, int qx,
                                              int qy, int u0, int nu, double *dst)
 {
@@ -142,10 +143,29 @@ __device__ __forceinline__ void smooth_block(QBlock &B, const QTileAt &T, int dx
                 plain &= div_plain(a[y], R);
             }
             if (!plain) {
+                bool rest = false;
 #pragma unroll
                 for (int y = 0; y < BY; ++y) {
                     const int x = (y + COL) & 1;
-                    if (!div_plain(a[y], Recip{B.b[y][x], B.rc[y][x]})) z[y] = div_by_rare(a[y], B.b[y][x], B.rc[y][x]);
+                    const Recip R{B.b[y][x], B.rc[y][x]};
+                    if (div_plain(a[y], R)) continue;
+                    if (!MEND) {
+                        z[y] = div_by_rare(a[y], R.b, R.y);
+                        continue;
+                    }
+                    // as div_by_rare, of the four cells without a call
+                    const double q = markstein(a[y] * 0x1p600, R), c = q * 0x1p-600;
+                    const bool zero = a[y] == 0.0;
+                    z[y] = zero ? a[y] * R.y : c;
+                    if ((__double2hiint(R.y) == 0) | (!zero & ((fabs(a[y]) >= 0x1p-918) | (fabs(fma(-c, 0x1p600, q)) == 0x1p-475))))
+                        rest = true;
+                }
+                if (rest) {
+#pragma unroll
+                    for (int y = 0; y < BY; ++y) {
+                        const int x = (y + COL) & 1;
+                        z[y] = div_by(a[y], Recip{B.b[y][x], B.rc[y][x]});
+                    }
                 }
             }
 #pragma unroll
@@ -216,7 +236,7 @@ __device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx
     if (!live) return;
     prepare_block(B, T, in.dx1, in.dy1, phi, qx, qy);
     __syncthreads();
-    smooth_block(B, T, in.dx1, in.dy1, npx, phi, qx, qy, u0, nu, in.dst);
+    smooth_block<false>(B, T, in.dx1, in.dy1, npx, phi, qx, qy, u0, nu, in.dst);
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -347,7 +367,7 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
             fetch(k + 2, blockIdx.x + (k + 2) * gridDim.x);
         }
         if (live)
-            smooth_block(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
+            smooth_block<true>(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
                          reinterpret_cast<double *>(now.b + (unsigned long long)(unsigned)(dir == 0 ? eq_tmp(now.e) : eq_field(now.e)) * now.sb));
         else
             __syncthreads();   // (phi has been read before it is written again)

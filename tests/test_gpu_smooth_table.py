@@ -48,6 +48,14 @@ def test_bitexact(nx, ny, ngrid, ncases, oracle_built):
     _compare([_cfg(nx, ny, ngrid, k) for k in range(ncases)], 3, (0, ncases // 2, ncases - 1), ngrid)
 
 
+def test_wide_obstacle(oracle_built):
+    """Values fall below the normal range deep inside (u, v by 1e-30 a cell, p' by 1e-60)."""
+    from mgfvm import configs
+    cfgs = [configs.small(32, 2, isolve=2, nfx=200, nfy=200, ig_obs=2, amuf=1.0 / (20.0 + k), obstacles=[(20, 80, 20, 80)])
+            for k in range(10)]
+    _compare(cfgs, 6, (0, 9), 2)
+
+
 def test_sizes(oracle_built):
     cfgs = [_cfg(*((256, 128, 3), (64, 64, 2), (128, 200, 3))[k % 3], k) for k in range(30)]
     _compare(cfgs, 2, (0, 1, 2, 27, 28, 29), 3)
