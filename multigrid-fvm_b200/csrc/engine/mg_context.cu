@@ -347,9 +347,34 @@ struct Builder {
     // half as many rounds, while a level of one round either way favours k_smooth's faster
     // units unless a single launch can take all of them.  (p' on two cases, 20 units: 256^2
     // 19.0 against 28.8 us, 128^2 17.7 against 14.4, 64^2 13.2 in one launch against 14.4.)
+    // (512-thread pair CTAs, where they all have an SM, small_blocks: about 1.3 a launch and
+    // 0.3 a unit, as the next launch's loads are under them.)
     struct QPlan {
         int chunks, tw, th, tiles;
     };
+    // the launches of a pair smoothing with CTAs of nt threads
+    struct PairShape {
+        int chunks, hmax, tile;   // hmax: units of the longest
+    };
+    PairShape pair_shape(int ig, int units, int nt, bool tmp_ok) const
+    {
+        const int most = (smooth_pairs_side(0, nt) - MIN_TILE) / 2;   // units that leave a MIN_TILE tile
+        const int cap = std::min(most, x->tune.smooth_units[ig] > 0 ? x->tune.smooth_units[ig] : MAX_UNITS);
+        int chunks = (units + cap - 1) / cap;
+        if ((chunks & 1) && units >= chunks + 1 && !tmp_ok) ++chunks;
+        const int hmax = (units + chunks - 1) / chunks;
+        return {chunks, hmax, smooth_pairs_side(hmax, nt)};
+    }
+    // Whether a pair smoothing runs CTAs of half the size: where every one of them then has an
+    // SM to itself, half the warps wait at a barrier and share its memory.  V-cycles of two
+    // 256^2 cases (their 64^2 level) 238 to 229 us, of three 304 x 112 ducts (152 x 56 and
+    // 76 x 28, Jacobi) 176 to 172, of a 64^2 channel 84 to 82; with two such CTAs an SM they
+    // were 1 to 4 us slower than with whole ones.
+    bool small_blocks(int ig, int neq, int tile) const
+    {
+        return tile >= MIN_TILE && !x->tune.smooth_threads[ig] && !x->tune.smooth_units[ig] && x->tune.smooth_tma[ig] != 2 &&
+               tiles(ig, tile) * x->ncases * neq <= SMS;
+    }
     bool smooth_q_plan(int ig, int neq, int units, bool tmp_ok, QPlan &best) const
     {
         if (x->sched.isolve != MGFVM_GAUSS_SEIDEL || x->tune.smooth_threads[ig] || x->tune.smooth_units[ig] ||
@@ -396,6 +421,8 @@ struct Builder {
             if (u <= MAX_UNITS && c <= (units + MAX_UNITS - 1) / MAX_UNITS + 1)
                 t_old = std::min(t_old, c * (0.3 + rounds(tile, tile, dummy) * (5.0 + 0.19 * u)));
         }
+        const PairShape p = pair_shape(ig, units, SMOOTH_BLOCK / 2, tmp_ok);
+        if (small_blocks(ig, neq, p.tile)) t_old = std::min(t_old, 0.3 + p.chunks * (1.3 + 0.3 * p.hmax));
         return t_best < t_old;
     }
     // Mixed precision's plan (k_smooth_q32), any number of launches; false where the tuning asks
@@ -528,13 +555,10 @@ struct Builder {
             return false;
         }
         const int tt = x->tune.smooth_threads[ig];
-        const int nt = tt == SMOOTH_BLOCK / 2 || tt == SMOOTH_BLOCK / 4 ? tt : SMOOTH_BLOCK;
-        const int most = (smooth_pairs_side(0, nt) - MIN_TILE) / 2;   // units that leave a MIN_TILE tile
-        const int cap = std::min(most, x->tune.smooth_units[ig] > 0 ? x->tune.smooth_units[ig] : MAX_UNITS);
-        int chunks = (units + cap - 1) / cap;
-        if ((chunks & 1) && units >= chunks + 1 && !tmp_ok) ++chunks;
-        const int hmax = (units + chunks - 1) / chunks;
-        const int tile = smooth_pairs_side(hmax, nt);
+        int nt = tt == SMOOTH_BLOCK / 2 || tt == SMOOTH_BLOCK / 4 ? tt : SMOOTH_BLOCK;
+        if (!tt && small_blocks(ig, neq, pair_shape(ig, units, SMOOTH_BLOCK / 2, tmp_ok).tile)) nt = SMOOTH_BLOCK / 2;
+        const PairShape shape = pair_shape(ig, units, nt, tmp_ok);
+        const int chunks = shape.chunks, hmax = shape.hmax, tile = shape.tile;
         const int side = tile + 2 * hmax;
         // TMA staging: a box one column wider than the region where it starts at an odd x
         const int bw = (side + 2) & ~1, bh = side;

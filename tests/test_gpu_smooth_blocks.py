@@ -29,7 +29,7 @@ def _cfg(nx, ny, ngrid, nswpm, nswpp, obstacles):
     (132, 138, 2, 2, 10, 48),     # 44 x 46: whole tiles at four units
     (134, 140, 2, 1, 3, 48),      # a cell more; two and six units
     (90, 94, 1, 3, 7, 64),        # six units of u, v, sc; fourteen of p'
-    (64, 64, 3, 2, 10, 4),        # one launch of twenty units
+    (64, 64, 3, 2, 10, 5),        # one launch of twenty units
     (300, 40, 2, 5, 1, 40),       # ten units of u, v, sc; wide and low
     (512, 256, 4, 2, 10, 2),
 ])
