@@ -1629,7 +1629,7 @@ __global__ void __launch_bounds__(BLOCK) k_endcycle(const CaseDev *__restrict__ 
     if ((int)blockIdx.x >= nb) return;
     int i, j;
     const bool cell = cell_at(d, blockIdx.x * blockDim.x + threadIdx.x, i, j);
-    end_of_cycle(C, ST, cell, i, j, nb);
+    end_of_cycle(C, ST, stops_on_error(C, ST.last_err), cell, i, j, nb);
 }
 
 // ------------------------------------------------- one-CTA coarse kernel

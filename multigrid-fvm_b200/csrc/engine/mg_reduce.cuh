@@ -59,12 +59,14 @@ static __device__ __forceinline__ void gather_partials(const double *partials, i
     block_sum<NV>(v);
 }
 
-// End of a V-cycle on the level-0 interior: relative change of u, v, sc and of p
-// with its mean removed against the previous cycle, the history entry, the stop
-// rule, and prev <- current.  p sums are shifted by the previous cycle's means so a
-// uniform pressure drift does not cancel catastrophically.
-// History entry and the reference's stop test (:247-248) when the fixed-point change is
-// not tracked: one thread per case.
+// The reference's stop test (:247-248) on the cycle's mass error, or that it is not finite.
+static __device__ __forceinline__ bool stops_on_error(const CaseDev &C, double err)
+{
+    return (C.stop_enabled != 0) & (!isfinite(err) | (err < C.convergence));
+}
+
+// History entry and that stop test when the fixed-point change is not tracked: one thread
+// per case.
 static __device__ __forceinline__ void end_of_cycle_err_only(const CaseDev &C, CaseState &ST)
 {
     const double err = ST.last_err;
@@ -76,21 +78,39 @@ static __device__ __forceinline__ void end_of_cycle_err_only(const CaseDev &C, C
     ST.ncyc = k + 1;
     const bool finite = isfinite(err);
     if (!finite) ST.status |= CASE_NONFINITE;
-    if (C.stop_enabled) {
-        if (!finite) ST.done = 1;
-        else if (err < C.convergence) { ST.done = 1; ST.status |= CASE_CONVERGED_REF; }
+    if (stops_on_error(C, err)) {
+        ST.done = 1;
+        if (finite) ST.status |= CASE_CONVERGED_REF;
     }
     ST.have_prev = 0;
 }
 
+// End of a V-cycle on the level-0 interior: relative change of u, v, sc and of p
+// with its mean removed against the previous cycle, the history entry, the stop
+// rule, and prev <- current.  p sums are shifted by the previous cycle's means so a
+// uniform pressure drift does not cancel catastrophically.
 // The fixed-point change (four norms over level 0 and their block reduction) is
 // computed only while a solve with fp_tol > 0 runs; otherwise the cycle only records
 // its mass error.
-// `cell`: this thread has level-0 cell (i, j); nb blocks take part.
-static __device__ __forceinline__ void end_of_cycle(const CaseDev &C, CaseState &ST, bool cell, int i, int j, int nb)
+// `cell`: this thread has level-0 cell (i, j); nb blocks take part.  `stops`: stops_on_error
+// of ST.last_err, read with the data the caller waits for anyway.
+static __device__ __forceinline__ void end_of_cycle(const CaseDev &C, CaseState &ST, bool stops, bool cell, int i, int j,
+                                                    int nb)
 {
     if (!(C.fp_tol > 0.0)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) end_of_cycle_err_only(C, ST);
+        if (!stops) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) end_of_cycle_err_only(C, ST);
+            return;
+        }
+        // Every block of this launch reads ST.done when it begins and does its part of the
+        // cycle unless it is set, so only the last one to get here may set it.  (Other cycles
+        // go without the counter.)
+        __syncthreads();
+        if (threadIdx.x != 0) return;
+        __threadfence();
+        if (atomicAdd(&C.counters[1], 1u) != (unsigned)nb - 1u) return;
+        C.counters[1] = 0;
+        end_of_cycle_err_only(C, ST);
         return;
     }
     const LevelDev &L = C.lv[0];

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(NT, 4) k_tile_prol(const CaseDev *__restrict__
     const bool active = mode_active(C, ig, mode) && j0 <= ny - 2;
     pdl_enter();
     if (!active) return;
-    const bool live = !st[blockIdx.y].done;
+    const bool live = !st[blockIdx.y].done, stops = END && stops_on_error(C, st[blockIdx.y].last_err);
     const int x = t % TX, y = t / TX, i = i0 + x, j = j0 + y, q = j * nx + i;
     const bool in = i <= nx - 2 && j <= ny - 2;
     double u = 0, v = 0, p = 0, sc = 0;
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(NT, 4) k_tile_prol(const CaseDev *__restrict__
         F.st(S_P, q, p);
         F.st(S_SC, q, sc);
     }
-    if (END && live) end_of_cycle(C, st[blockIdx.y], in, i, j, tiles_of(nx - 2, ny - 2));
+    if (END && live) end_of_cycle(C, st[blockIdx.y], stops, in, i, j, tiles_of(nx - 2, ny - 2));
 }
 
 cudaError_t launch_tile(const Launch &X, const CaseDev *dc, CaseState *ds, const Sched &S, cudaStream_t st)
