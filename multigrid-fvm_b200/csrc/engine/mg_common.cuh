@@ -92,6 +92,7 @@ struct CaseDev {
 // The part of a case that kernels write.
 struct CaseState {
     int done;           // stop rule fired; every kernel skips this case
+    int gone;           // `done`, as the level-0 update of a later cycle has seen it
     int status;         // enum CaseStatus bits
     int ncyc;           // cycles recorded in the history
     int have_prev;      // level-0 state of a previous cycle is in S_PREV_*

@@ -1123,7 +1123,7 @@ int set_controls(mgfvm_ctx *x, int stop, double fp_tol)
         C.stop_enabled = stop;
         C.fp_tol = fp_tol;
     }
-    for (CaseState &S : x->hs) S.done = 0;
+    for (CaseState &S : x->hs) S.done = S.gone = 0;
     return push(x);
 }
 

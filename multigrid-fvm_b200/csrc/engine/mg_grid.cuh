@@ -51,6 +51,17 @@ static __device__ __forceinline__ void pdl_enter()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Whether a launch of this mode may leave a case out, read before it waits for the launch
+// before it: `done` is set by the launch that ends a cycle, which is directly followed by
+// the first launch of level 0 (that takes `gone`, or reads `done` after its wait) or by an
+// op.  The blocks of a stopped case end there, before they load anything: a cycle of 64
+// stopped 256^2 cases takes 0.28 ms against 1.52 where the flag was read along with the
+// data, of two 60 us against 115 (a running one 2.29 ms and 228 us).
+static __device__ __forceinline__ bool stopped_before(const CaseState &S, int mode)
+{
+    return (S.done != 0) & (mode > M_OP_C);
+}
+
 // Launch `k` on `st`, with programmatic stream serialization when `pdl` (the kernel
 // may then be scheduled while its predecessor runs; it waits in pdl_enter()).
 template <typename... KP, typename... A>

@@ -215,6 +215,13 @@ __global__ void __launch_bounds__(BLOCK) k_update(const CaseDev *__restrict__ cs
     const FastLevel L = fast_level(C.lv[ig]);
     const Fast io{L};
     const int nx = L.npx, n = (nx - 2) * (L.npy - 2), t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        if (ig == 0 && t == 0) st[blockIdx.y].gone = 1;   // for the level-0 assembly
+        return;
+    }
     const bool out = (fuse & 1) && C.ibc_xp == 4, active = mode_active(C, ig, mode);
     int i, j;
     const bool cell = active && cell_at({1, 1, nx - 2, L.npy - 2}, t, i, j);
@@ -254,7 +261,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(const CaseDev *__restrict__ cs
 // with bit 2, the smoother is Jacobi.
 // EARLY: the previous launch is a smoother, which writes none of the coefficients'
 // operands (areas, apu, apv, tag): the coefficients are formed before waiting for it,
-// u and v read after (a finished case, ST.done, set at the end of a cycle, forms nothing).
+// u and v read after.
 template <bool EARLY>
 __global__ void __launch_bounds__(BLOCK) k_mass_coefp(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int reduce,
                                                       int flags)
@@ -264,6 +271,12 @@ __global__ void __launch_bounds__(BLOCK) k_mass_coefp(const CaseDev *__restrict_
     const FastLevel L = fast_level(C.lv[ig]);
     const Fast io{L};
     const int n = (L.npx - 2) * (L.npy - 2), nb = (n + blockDim.x - 1) / blockDim.x;
+    const bool stopped = stopped_before(ST, mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && (int)blockIdx.x < nb;
     int i, j;
     const bool cell = active && cell_at({1, 1, L.npx - 2, L.npy - 2}, blockIdx.x * blockDim.x + threadIdx.x, i, j);
@@ -523,8 +536,7 @@ __device__ __forceinline__ void pair_units(const double (&c)[2][NCOEF], const Re
 // writes).  Every cell update is the reference's formula on the same neighbour values,
 // so the result is bit-identical to sweeping the whole level unit by unit.
 // EARLY: the coefficients were written before the previous launch (a later launch of a
-// smoothing split in several), so they are read before waiting for it (a finished
-// case, ST.done, set at the end of a cycle, loads nothing).
+// smoothing split in several), so they are read before waiting for it.
 template <int ISOLVE, int NT, bool EARLY>
 __global__ void __launch_bounds__(NT, SMOOTH_BLOCK / NT) k_smooth(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int mask, int u0, int nu,
                                                          int dir, int tile)
@@ -536,6 +548,12 @@ __global__ void __launch_bounds__(NT, SMOOTH_BLOCK / NT) k_smooth(const CaseDev 
     const Fast io{L};
     const int e = nth_eq(mask, blockIdx.z);
     PairTile P;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const int g = mode_active(C, ig, mode)
                       ? pair_tile<!JAC>(Dom{1, 1, L.npx - (e == EQ_U ? 3 : 2), L.npy - (e == EQ_V ? 3 : 2)}, L.npx, nu, tile, P, blockIdx.x)
                       : 1;
@@ -963,6 +981,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(NT, 1)
     CaseState &ST = st[blockIdx.y];
     const FastLevel L = fast_level(C.lv[ig]);
     const Fast io{L};
+    if (!(ig == 0 && mode == M_DOWN) && stopped_before(ST, mode)) {   // the same for the three CTAs
+        pdl_enter();
+        return;
+    }
     const bool on = mode_active(C, ig, mode);
     const int W = L.npx, H = L.npy, n = W * H, r = blockIdx.x, t = threadIdx.x;
     const int e = r == 0 ? EQ_U : r == 1 ? EQ_V : EQ_SC, field = eq_field(e);

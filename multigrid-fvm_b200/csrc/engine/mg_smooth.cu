@@ -276,9 +276,9 @@ __device__ __forceinline__ void copy_async16(void *to, const void *from)
 // gridDim.x-th of the table `tab`.  While a tile is smoothed, one thread has the next one's
 // coefficients and field copied (TMA) into shared memory, from where the threads fetch their
 // blocks, and the table entry after that: only the first tile's way from memory is waited
-// for.  `maps` has each case's two tensor maps with a box of bw x bh cells (even bw: a box
-// starts at an even column).  A copy that does not land within `polls` polls:
-// CASE_WAIT_TIMEOUT, as k_smooth_tma.
+// for.  Tiles of cases that have stopped are left out.  `maps` has each case's two tensor
+// maps with a box of bw x bh cells (even bw: a box starts at an even column).  A copy that
+// does not land within `polls` polls: CASE_WAIT_TIMEOUT, as k_smooth_tma.
 // A tile takes 3.5 us and 0.37 a unit here, 4.9 and 0.37 with a CTA a tile (k_smooth_q),
 // bound by the copies (25 MB a round of CTAs) and the fetch that waits for them.  Level 0 of
 // 64 256^2 obstacle cases: five p' units 88 us against 111, four of u, v, sc 225 against 300;
@@ -292,17 +292,31 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
 {
     extern __shared__ __align__(128) double ahead[];   // coefficients, then the field
     __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
-    __shared__ QTile entry[3];   // of tile k (its number in this CTA), in k % 3
-    __shared__ int there[3];     // there is a tile k
+    constexpr int WARPS = SMOOTH_Q_THREADS / 32;
+    __shared__ QTile entry[3];   // of the s-th tile this CTA takes, in s % 3
+    __shared__ int there[3];     // there is one
+    __shared__ int last;         // which of the CTA's share of the table was fetched last
+    __shared__ unsigned running[WARPS];   // bit k of these: the k-th of that share is of a case that has not stopped
     __shared__ __align__(8) unsigned long long mbar;
     double *phi = smq + 2 * QX;
     const int t = threadIdx.x, qx = t % QX, qy = t / QX, box = bw * bh, fbox = ahead_field(box);
     const unsigned bar = smem_addr(&mbar);
-    auto fetch = [&](int k, int n) {   // the entry of tile k, number n
-        there[k % 3] = n < ntab;
+    auto fetch = [&](int s) {    // the s-th tile's entry: the next of a case that runs
+        int k = last + 1;
+        while (k < 32 * WARPS) {
+            const unsigned w = running[k / 32] >> (k % 32);
+            if (w) {
+                k += __ffs(w) - 1;
+                break;
+            }
+            k = (k / 32 + 1) * 32;
+        }
+        last = k;
+        const int n = blockIdx.x + k * gridDim.x;
+        there[s % 3] = n < ntab;
         if (n >= ntab) return;
         for (int c = 0; c < (int)sizeof(QTile) / 16; ++c)
-            copy_async16(reinterpret_cast<char *>(&entry[k % 3]) + 16 * c, reinterpret_cast<const char *>(tab + n) + 16 * c);
+            copy_async16(reinterpret_cast<char *>(&entry[s % 3]) + 16 * c, reinterpret_cast<const char *>(tab + n) + 16 * c);
     };
     auto first_cell = [&](int n0, int n) { return max(1 + n0 * n - nu, 0) & ~1; };
     auto coefs = [&](const QTile &N) {
@@ -319,8 +333,15 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         entry[0] = tab[blockIdx.x];
+        last = 0;
         if (EARLY) coefs(entry[0]);
-        fetch(1, blockIdx.x + gridDim.x);
+    }
+    // the first tile is on its way without a look at its case; of the rest, those of cases
+    // that have stopped are left out (beyond the first 384 they are taken, and not smoothed)
+    {
+        const int n = blockIdx.x + t * gridDim.x;
+        const unsigned w = __ballot_sync(0xffffffffu, n < ntab && !st[tab[n].icase].done);
+        if ((t & 31) == 0) running[t / 32] = w;
     }
     pdl_enter();
     if (t == 0) {
@@ -328,14 +349,15 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         field(entry[0]);
     }
     __syncthreads();
-    for (int k = 0;; ++k) {
-        const QTile now = entry[k % 3];
+    if (t == 0) fetch(1);
+    for (int s = 0;; ++s) {
+        const QTile now = entry[s % 3];
         const int dx1 = now.npx - (now.e == EQ_U ? 3 : 2), dy1 = now.npy - (now.e == EQ_V ? 3 : 2);
         const QTileAt T = tile_at(dx1, dy1, now.tx, now.ty, tw, th, nu, qx, qy);
         const bool live = !st[now.icase].done;
         QBlock B;
         clear_block(B);
-        const bool landed = mbar_wait(bar, k & 1, polls);
+        const bool landed = mbar_wait(bar, s & 1, polls);
         auto load = [&](int at, double (&a)[BY][BX]) {
 #pragma unroll
             for (int y = 0; y < BY; ++y)
@@ -353,18 +375,18 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         load(CK_SU * box, B.su);
         load(fbox, B.v);
         prepare_block(B, T, dx1, dy1, phi, qx, qy);
-        if (t == 0) asm volatile("cp.async.wait_all;" ::: "memory");   // entry k + 1
+        if (t == 0) asm volatile("cp.async.wait_all;" ::: "memory");   // entry s + 1
         // one decision for the whole block; after it, `ahead` has been read
         if (!__syncthreads_and(landed)) {
             if (t == 0) atomicOr(&st[now.icase].status, (int)CASE_WAIT_TIMEOUT);
-            mbar_wait(bar, k & 1, TMA_WAIT_POLLS);
+            mbar_wait(bar, s & 1, TMA_WAIT_POLLS);
             return;
         }
-        const bool more = there[(k + 1) % 3];
+        const bool more = there[(s + 1) % 3];
         if (t == 0 && more) {
-            coefs(entry[(k + 1) % 3]);
-            field(entry[(k + 1) % 3]);
-            fetch(k + 2, blockIdx.x + (k + 2) * gridDim.x);
+            coefs(entry[(s + 1) % 3]);
+            field(entry[(s + 1) % 3]);
+            fetch(s + 2);
         }
         if (live)
             smooth_block<true>(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
@@ -396,6 +418,12 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
     in.src = io.at(dir == 1 ? eq_tmp(e) : eq_field(e));
     in.dst = io.at(dir == 0 ? eq_tmp(e) : eq_field(e));
     const int txn = max(1, (in.dx1 + tw - 1) / tw), tyn = (in.dy1 + th - 1) / th;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && in.dx1 >= 1 && in.dy1 >= 1 && (int)blockIdx.x < txn * tyn;
     smooth_q_tile<EARLY>(in, active, blockIdx.x % txn, blockIdx.x / txn, tw, th, u0, nu, [&]() {
         pdl_enter();
@@ -434,6 +462,12 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 2)
     const int e = nth_eq(mask, blockIdx.z), npx = L.npx, t = threadIdx.x, qx = t % QX, qy = t / QX;
     const int dx1 = npx - (e == EQ_U ? 3 : 2), dy1 = L.npy - (e == EQ_V ? 3 : 2);
     const int txn = max(1, (dx1 + tw - 1) / tw), tx = blockIdx.x % txn, ty = blockIdx.x / txn;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && dx1 >= 1 && dy1 >= 1 && ty * th < dy1;
     const bool first = (flags & 1) != 0, last = (flags & 2) != 0;
     const QTileAt T = tile_at(dx1, dy1, tx, ty, tw, th, nu, qx, qy);

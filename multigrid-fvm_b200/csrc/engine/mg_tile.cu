@@ -49,6 +49,14 @@ __global__ void __launch_bounds__(NT, 3)
     const Fast io{L};
     const int nx = L.npx, ny = L.npy, t = threadIdx.x, txn = max(1, (nx + TX - 1) / TX);
     const int i0 = (blockIdx.x % txn) * TX, j0 = (blockIdx.x / txn) * TY;
+    // (the level-0 assembly comes right after the launch that sets `done`, so it takes `gone`)
+    const bool first = !REST && ig == 0 && mode == M_DOWN;
+    const bool stopped = first ? st[blockIdx.y].gone != 0 : stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && j0 < ny;
     if (REST && !mode_active(C, ig + 1, M_DOWN)) what = 0;
     const bool assemble = !REST || what != 0, sc_out = (what & A_SC_OUTFLOW) && C.ibc_xp == 4;
@@ -203,8 +211,15 @@ __global__ void __launch_bounds__(NT, 3)
     const CaseDev &C = cs[blockIdx.y];
     const FastLevel L = fast_level(C.lv[ig]), LK = fast_level(C.lv[ig + 1]);
     const Fast F{L}, K{LK};
+    begin_loads(C, LK);
     const int nx = L.npx, ny = L.npy, t = threadIdx.x, txn = max(1, (nx - 2 + TX - 1) / TX);
     const int i0 = 1 + (blockIdx.x % txn) * TX, j0 = 1 + (blockIdx.x / txn) * TY;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && j0 <= ny - 2;
     pdl_enter();
     if (!active) return;
@@ -363,8 +378,15 @@ __global__ void __launch_bounds__(NT, 4) k_tile_prol(const CaseDev *__restrict__
     const CaseDev &C = cs[blockIdx.y];
     const FastLevel L = fast_level(C.lv[ig]), LK = fast_level(C.lv[ig + 1]);
     const Fast F{L}, K{LK};
+    begin_loads(C, LK);
     const int nx = L.npx, ny = L.npy, nxc = LK.npx, nyc = LK.npy, t = threadIdx.x, txn = max(1, (nx - 2 + TX - 1) / TX);
     const int i0 = 1 + (blockIdx.x % txn) * TX, j0 = 1 + (blockIdx.x / txn) * TY;
+    const bool stopped = stopped_before(st[blockIdx.y], mode);
+    begin_loads(C, L);
+    if (stopped) {
+        pdl_enter();
+        return;
+    }
     const bool active = mode_active(C, ig, mode) && j0 <= ny - 2;
     pdl_enter();
     if (!active) return;
