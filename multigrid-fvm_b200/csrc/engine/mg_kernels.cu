@@ -2197,11 +2197,12 @@ __global__ void __launch_bounds__(BLOCK) r_jacobi(const double *__restrict__ aw,
 }
 
 // Jacobi by tiles: `nu` sweeps of the tile plus a halo of one cell a sweep in shared memory
-// (k_smooth on a caller's level), from src to dst.
+// (k_smooth on a caller's level), from src to dst, with `ring` the boundary ring too (which
+// the caller's own field has already, and is not written there).
 __global__ void __launch_bounds__(SMOOTH_BLOCK, 1)
     r_jacobi_tile(const double *__restrict__ aw, const double *__restrict__ ae, const double *__restrict__ as,
                   const double *__restrict__ an, const double *__restrict__ ap, const double *__restrict__ su,
-                  const double *src, double *dst, int npx, int wi, int wj, int nu, int tile)
+                  const double *src, double *dst, bool ring, int npx, int wi, int wj, int nu, int tile)
 {
     extern __shared__ double sm[];
     PairTile P;
@@ -2234,7 +2235,7 @@ __global__ void __launch_bounds__(SMOOTH_BLOCK, 1)
     pair_units<MGFVM_JACOBI>(c, R, v, lim[0], lim[1], k2[0], k2[1], 0, nu, W, phi, phi2);
 #pragma unroll
     for (int x = 0; x < 2; ++x)
-        if (out[x]) dst[g2[x]] = v[x];
+        if (out[x] && (ring || lim[x] >= 0)) dst[g2[x]] = v[x];
 }
 
 __global__ void __launch_bounds__(BLOCK) r_copy(const double *src, double *dst, int npx, int nx, int ny)
@@ -2344,7 +2345,7 @@ cudaError_t raw_jacobi(const double *aw, const double *ae, const double *as, con
                 const double *src = (c & 1) ? scratch : phi;
                 double *dst = (c & 1) || chunks == 1 ? phi : scratch;
                 const cudaError_t e = launch_k(c > 0, r_jacobi_tile, grid, block, 2 * cells * (int)sizeof(double), s, aw,
-                                               ae, as, an, ap, su, src, dst, npx, wi, wj, nu, tile);
+                                               ae, as, an, ap, su, src, dst, dst != phi, npx, wi, wj, nu, tile);
                 if (e != cudaSuccess) return e;
             }
             return cudaSuccess;

@@ -47,6 +47,7 @@ struct QIn {
     const double *co[NCOEF], *src;
     double *dst;
     int npx, dx1, dy1;
+    bool ring;  // dst takes the boundary ring too (it has it already where it is a caller's own field)
     bool vec;   // a block row's two cells may be loaded together (16-byte aligned)
 };
 
@@ -110,10 +111,10 @@ __device__ __forceinline__ void prepare_block(QBlock &B, const QTileAt &T, int d
     }
 }
 // The units u0 .. u0 + nu - 1 (each between barriers; one precedes the first), then the tile,
-// plus the boundary ring where it touches it, to dst.
+// with `ring` plus the boundary ring where it touches it, to dst.
 template <bool MEND>
 __device__ __forceinline__ void smooth_block(QBlock &B, const QTileAt &T, int dx1, int dy1, int npx, double *phi, int qx,
-                                             int qy, int u0, int nu, double *dst)
+                                             int qy, int u0, int nu, double *dst, bool ring)
 {
     const int i = T.i, j = T.j, x0 = T.x0, x1 = T.x1, y0 = T.y0, y1 = T.y1;
     for (int h = 1; h <= nu; ++h) {
@@ -181,8 +182,8 @@ __device__ __forceinline__ void smooth_block(QBlock &B, const QTileAt &T, int dx
         else unit(std::integral_constant<int, 1>{});
         __syncthreads();
     }
-    const int ox0 = x0 == 1 ? 0 : x0, ox1 = x1 == dx1 ? x1 + 1 : x1;
-    const int oy0 = y0 == 1 ? 0 : y0, oy1 = y1 == dy1 ? y1 + 1 : y1;
+    const int ox0 = ring && x0 == 1 ? 0 : x0, ox1 = ring && x1 == dx1 ? x1 + 1 : x1;
+    const int oy0 = ring && y0 == 1 ? 0 : y0, oy1 = ring && y1 == dy1 ? y1 + 1 : y1;
     if (T.mine) {
 #pragma unroll
         for (int y = 0; y < BY; ++y)
@@ -236,7 +237,7 @@ __device__ __forceinline__ void smooth_q_tile(const QIn &in, bool active, int tx
     if (!live) return;
     prepare_block(B, T, in.dx1, in.dy1, phi, qx, qy);
     __syncthreads();
-    smooth_block<false>(B, T, in.dx1, in.dy1, npx, phi, qx, qy, u0, nu, in.dst);
+    smooth_block<false>(B, T, in.dx1, in.dy1, npx, phi, qx, qy, u0, nu, in.dst, in.ring);
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         }
         if (live)
             smooth_block<true>(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
-                         reinterpret_cast<double *>(now.b + (unsigned long long)(unsigned)(dir == 0 ? eq_tmp(now.e) : eq_field(now.e)) * now.sb));
+                         reinterpret_cast<double *>(now.b + (unsigned long long)(unsigned)(dir == 0 ? eq_tmp(now.e) : eq_field(now.e)) * now.sb), true);
         else
             __syncthreads();   // (phi has been read before it is written again)
         if (!more) return;
@@ -412,6 +413,7 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
     in.npx = L.npx;
     in.dx1 = L.npx - (e == EQ_U ? 3 : 2);
     in.dy1 = L.npy - (e == EQ_V ? 3 : 2);
+    in.ring = true;
     in.vec = (L.npx & 1) == 0;
 #pragma unroll
     for (int k = 0; k < NCOEF; ++k) in.co[k] = io.at(co_slot(e, k));
@@ -653,6 +655,7 @@ cudaError_t raw_smooth_q(const double *const *co, double *phi, double *tmp, int 
         const int nu = units / chunks + (c < units % chunks ? 1 : 0);
         in.src = (c & 1) ? tmp : phi;
         in.dst = (c & 1) || chunks == 1 ? phi : tmp;
+        in.ring = in.dst != phi;
         const cudaError_t e = c == 0 ? launch_k(false, r_smooth_q<false>, dim3(tiles), SMOOTH_Q_THREADS, 0, st, in, u0, nu, tw, th)
                                      : launch_k(true, r_smooth_q<true>, dim3(tiles), SMOOTH_Q_THREADS, 0, st, in, u0, nu, tw, th);
         if (e != cudaSuccess) return e;
