@@ -434,12 +434,26 @@ int mgfvm_jacobi_f64(const double *aw, const double *ae, const double *as,
                      int nsw, void *stream);
 
 /* Red-black Gauss-Seidel, `nsw` sweeps of a red pass ((i+j) even) then a black
- * pass, in place, phi <- (sum a_nb phi_nb + su) / ap.  Replaces solvergs(),
- * Version-6-26-04.c:1297-1351. */
+ * pass, in place, phi <- (sum a_nb phi_nb + su) / ap; the cells round i in [1, nx-1],
+ * j in [1, ny-1] are read only.  Replaces solvergs(), Version-6-26-04.c:1297-1351.
+ * Extents larger than one tile (52 x 54 cells) go through npx*npy doubles of device
+ * memory that the call takes from the library's memory pool of the current device and
+ * gives back, both in stream order (the pool, which the contexts share, keeps up to
+ * 4 GiB of what was given back until the process ends).  On a stream that is being
+ * captured, and where the device has no room, a launch a half-sweep does the same in
+ * place: the same bits, up to five times slower. */
 int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as,
                    const double *an, const double *ap, const double *su,
                    double *phi, int npx, int npy, int nx, int ny, int nsw,
                    void *stream);
+
+/* The same for callers that cannot allocate device memory (see
+ * mgfvm_masserror_f64_noalloc): takes none and enters no allocator.  No counterpart in
+ * the reference. */
+int mgfvm_rbgs_f64_noalloc(const double *aw, const double *ae, const double *as,
+                           const double *an, const double *ap, const double *su,
+                           double *phi, int npx, int npy, int nx, int ny, int nsw,
+                           void *stream);
 
 /* Mass residual: su = -div, pp = 0 on the interior and *err_out (device) =
  * sum |div|, reduced in a fixed order through `partials` (caller-owned device

@@ -2131,8 +2131,9 @@ int mgfvm_jacobi_f64(const double *aw, const double *ae, const double *as, const
     return MGFVM_OK;
 }
 
-int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as, const double *an, const double *ap,
-                   const double *su, double *phi, int npx, int npy, int nx, int ny, int nsw, void *stream)
+// `buffer`: device memory may be taken for the duration of the call
+static int rbgs(const double *aw, const double *ae, const double *as, const double *an, const double *ap,
+                const double *su, double *phi, int npx, int npy, int nx, int ny, int nsw, void *stream, bool buffer)
 {
     const void *p[] = {aw, ae, as, an, ap, su, phi};
     RC(check_raw(p, 7, npx, npy, nx, ny));
@@ -2142,18 +2143,18 @@ int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as, const d
         // 4.1 us, 7.8 us a million cells where that is more (12 sweeps of 90 x 70: 100 us
         // against 20 by tiles; two of 1024 x 1024: 33 against 35).  Several tile launches go
         // through a buffer taken from the device's pool in stream order, which a stream that
-        // is being captured (or a full device) does without.
+        // is being captured (or a full device, or a caller that wants none) does without.
         const int wi = nx - 1, wj = ny - 1;
         int chunks = 0, tw = 0, th = 0;
         const double *co[] = {aw, ae, as, an, ap, su};
         const double plain = 2.0 * nsw * std::max(4.1, 7.8e-6 * wi * wj);
         const double t = raw_q_plan(wi, wj, 2 * nsw, chunks, tw, th);
-        if (t < plain) {
+        if (t < plain && chunks == 1) {
+            CK(raw_smooth_q(co, phi, phi, npx, wi, wj, 2 * nsw, 1, tw, th, (cudaStream_t)stream));
+            return MGFVM_OK;
+        }
+        if (t < plain && buffer) {
             cudaStream_t st = (cudaStream_t)stream;
-            if (chunks == 1) {
-                CK(raw_smooth_q(co, phi, phi, npx, wi, wj, 2 * nsw, 1, tw, th, st));
-                return MGFVM_OK;
-            }
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
             cudaStreamCaptureMode relaxed = cudaStreamCaptureModeRelaxed;   // (of other threads' streams)
             int dev = 0;
@@ -2162,8 +2163,10 @@ int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as, const d
             cudaError_t e = cudaStreamIsCapturing(st, &cap);
             if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone && cudaGetDevice(&dev) == cudaSuccess) {
                 cudaMemPool_t mp = device_pool(dev);
-                if (!mp || cudaMallocFromPoolAsync(&tmp, sizeof(double) * (size_t)npx * npy, mp, st) != cudaSuccess)
+                if (mp && cudaMallocFromPoolAsync(&tmp, sizeof(double) * (size_t)npx * npy, mp, st) != cudaSuccess) {
                     tmp = nullptr;
+                    cudaMemPoolTrimTo(mp, 0);   // (what it grew by before it refused)
+                }
             }
             if (tmp) {
                 e = raw_smooth_q(co, phi, (double *)tmp, npx, wi, wj, 2 * nsw, chunks, tw, th, st);
@@ -2179,6 +2182,18 @@ int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as, const d
     }
     CK(mg::raw_rbgs(aw, ae, as, an, ap, su, phi, npx, npy, nx, ny, nsw, (cudaStream_t)stream));
     return MGFVM_OK;
+}
+
+int mgfvm_rbgs_f64(const double *aw, const double *ae, const double *as, const double *an, const double *ap,
+                   const double *su, double *phi, int npx, int npy, int nx, int ny, int nsw, void *stream)
+{
+    return rbgs(aw, ae, as, an, ap, su, phi, npx, npy, nx, ny, nsw, stream, true);
+}
+
+int mgfvm_rbgs_f64_noalloc(const double *aw, const double *ae, const double *as, const double *an, const double *ap,
+                           const double *su, double *phi, int npx, int npy, int nx, int ny, int nsw, void *stream)
+{
+    return rbgs(aw, ae, as, an, ap, su, phi, npx, npy, nx, ny, nsw, stream, false);
 }
 
 size_t mgfvm_masserror_scratch_doubles(int npx, int npy)
