@@ -261,9 +261,10 @@ __global__ void __launch_bounds__(BLOCK) k_update(const CaseDev *__restrict__ cs
 // with bit 2, the smoother is Jacobi.
 // EARLY: the previous launch is a smoother, which writes none of the coefficients'
 // operands (areas, apu, apv, tag): the coefficients are formed before waiting for it,
-// u and v read after.
+// u and v read after.  Five blocks an SM: with 56 registers, four, 40 cases of 64^2 take a
+// wave more (a V-cycle of one level 77.9 us against 75.4).
 template <bool EARLY>
-__global__ void __launch_bounds__(BLOCK) k_mass_coefp(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int reduce,
+__global__ void __launch_bounds__(BLOCK, EARLY ? 5 : 4) k_mass_coefp(const CaseDev *__restrict__ cs, CaseState *st, int ig, int mode, int reduce,
                                                       int flags)
 {
     const CaseDev &C = cs[blockIdx.y];

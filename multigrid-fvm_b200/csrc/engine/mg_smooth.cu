@@ -293,31 +293,32 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
 {
     extern __shared__ __align__(128) double ahead[];   // coefficients, then the field
     __shared__ double smq[2 * QX * (SMOOTH_Q_ROWS + 2)];
-    constexpr int WARPS = SMOOTH_Q_THREADS / 32;
+    constexpr int KEPT = SMOOTH_Q_THREADS - 32;   // flags
     __shared__ QTile entry[3];   // of the s-th tile this CTA takes, in s % 3
     __shared__ int there[3];     // there is one
     __shared__ int last;         // which of the CTA's share of the table was fetched last
-    __shared__ unsigned running[WARPS];   // bit k of these: the k-th of that share is of a case that has not stopped
+    __shared__ unsigned running[KEPT / 32];   // bit k of these: the k-th of that share is of a case that has not stopped
     __shared__ __align__(8) unsigned long long mbar;
     double *phi = smq + 2 * QX;
     const int t = threadIdx.x, qx = t % QX, qy = t / QX, box = bw * bh, fbox = ahead_field(box);
     const unsigned bar = smem_addr(&mbar);
-    auto fetch = [&](int s) {    // the s-th tile's entry: the next of a case that runs
-        int k = last + 1;
-        while (k < 32 * WARPS) {
-            const unsigned w = running[k / 32] >> (k % 32);
-            if (w) {
-                k += __ffs(w) - 1;
-                break;
-            }
-            k = (k / 32 + 1) * 32;
-        }
+    // the s-th tile's entry, the share's k-th
+    auto fetch = [&](int s, int k) {
         last = k;
         const int n = blockIdx.x + k * gridDim.x;
         there[s % 3] = n < ntab;
         if (n >= ntab) return;
         for (int c = 0; c < (int)sizeof(QTile) / 16; ++c)
             copy_async16(reinterpret_cast<char *>(&entry[s % 3]) + 16 * c, reinterpret_cast<const char *>(tab + n) + 16 * c);
+    };
+    // the first of the share's from the k-th on whose case runs
+    auto next = [&](int k) {
+        while (k < KEPT) {
+            const unsigned w = running[k / 32] >> (k % 32);
+            if (w) return k + __ffs(w) - 1;
+            k = (k / 32 + 1) * 32;
+        }
+        return k;
     };
     auto first_cell = [&](int n0, int n) { return max(1 + n0 * n - nu, 0) & ~1; };
     auto coefs = [&](const QTile &N) {
@@ -334,23 +335,28 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         entry[0] = tab[blockIdx.x];
-        last = 0;
         if (EARLY) coefs(entry[0]);
+        fetch(1, 1);
     }
     // the first tile is on its way without a look at its case; of the rest, those of cases
-    // that have stopped are left out (beyond the first 384 they are taken, and not smoothed)
-    {
-        const int n = blockIdx.x + t * gridDim.x;
-        const unsigned w = __ballot_sync(0xffffffffu, n < ntab && !st[tab[n].icase].done);
-        if ((t & 31) == 0) running[t / 32] = w;
+    // that have stopped are left out (beyond the flags kept they are taken, and not smoothed)
+    bool stopped = false;
+    if (t >= 32) {
+        const int n = blockIdx.x + (t - 32) * gridDim.x;
+        stopped = n < ntab && st[tab[n].icase].done;
+        const unsigned w = __ballot_sync(0xffffffffu, n < ntab && !stopped);
+        if ((t & 31) == 0) running[t / 32 - 1] = w;
     }
     pdl_enter();
     if (t == 0) {
         if (!EARLY) coefs(entry[0]);
         field(entry[0]);
     }
-    __syncthreads();
-    if (t == 0) fetch(1);
+    const bool some = __syncthreads_or(stopped);   // tiles may have to be left out
+    if (some && t == 0 && next(1) != 1) {          // (not the one fetched beforehand)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fetch(1, next(1));
+    }
     for (int s = 0;; ++s) {
         const QTile now = entry[s % 3];
         const int dx1 = now.npx - (now.e == EQ_U ? 3 : 2), dy1 = now.npy - (now.e == EQ_V ? 3 : 2);
@@ -387,7 +393,7 @@ __global__ void __launch_bounds__(SMOOTH_Q_THREADS, 1)
         if (t == 0 && more) {
             coefs(entry[(s + 1) % 3]);
             field(entry[(s + 1) % 3]);
-            fetch(s + 2);
+            fetch(s + 2, some ? next(last + 1) : s + 2);
         }
         if (live)
             smooth_block<true>(B, T, dx1, dy1, now.npx, phi, qx, qy, u0, nu,
