@@ -189,8 +189,9 @@ typedef struct mgfvm_tuning {
                                               rows, halo rows exchanged in distributed
                                               shared memory; FP64 in either precision):
                                               the whole visit in one launch: 2 yes, 1 no,
-                                              0 yes in large batches (64 cases; 32 in
-                                              mixed precision) of one size at the level */
+                                              0 yes in batches of one size at the level
+                                              where that is expected to be the faster
+                                              (mixed precision: from 32 cases on)     */
     int coarse_cluster;                    /* every level from the first one a CTA per case
                                               holds down to the coarsest, with the
                                               transfers into and out of it, as one launch

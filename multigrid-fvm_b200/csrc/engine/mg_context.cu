@@ -99,6 +99,7 @@ struct mgfvm_ctx {
     // and the tiles of its K_SMOOTH_Q launches that have more of them than SMs
     std::vector<QTile> htiles;
     QTile *dtiles = nullptr;
+    std::map<std::tuple<int, int, int>, int> band_slots;   // band_clusters by (G, block, smem)
     std::vector<int> tail0;                   // per case: first one-CTA-kernel level chosen at creation
     std::vector<void *> pooled;               // buffers taken from the device's memory pool
     // the last mgfvm_adjoint: per case J and its gradient (nfy inlet faces, amuf, prsc)
@@ -321,16 +322,48 @@ struct Builder {
         return mode != M_OP && x->sched.nswpp > 0 && t != 1 &&
                (isolve == MGFVM_JACOBI || isolve == MGFVM_GAUSS_SEIDEL) && !whole_level(ig, mx, my) &&
                band_level(ig, G, blk, smem) &&
-               (t == 2 || (band_default(G) && one_size(ig, mx, my)));
+               (t == 2 || (one_size(ig, mx, my) && band_default(ig, G, blk, smem)));
     }
-    // The sizes of batch at which band visits of a G-CTA level are the faster ones.  FP64:
-    // only where a pair of CTAs holds the level (66^2 of a 256^2 case: 64 cases 2.32 ms per
-    // V-cycle against 2.34 with tiles, 128 4.52 against 4.53, 32 1.28 against 1.24).
-    // Mixed precision, whose tiles are FP32 and slower here: BAND_MIN_CASES.
-    bool band_default(int G) const
+    // Whether band visits of a level all cases have at one size are expected to be the faster
+    // ones.  Mixed precision, whose tiles are FP32: from BAND_MIN_CASES on.  FP64: by the time
+    // of a visit in microseconds, fitted to single levels of 40 x 56 to 256 x 60 cells, 8 to
+    // 256 cases and three sweep counts.  A wave of as many clusters as the device holds takes
+    // some 57 and one a unit (a quarter less with half the threads); tiles take time in
+    // proportion to the cells with Jacobi, and with Gauss-Seidel that of their plan and of the
+    // assembly, the residual and the update.  (Bands against tiles, 2 + 10 sweeps: Jacobi, 128
+    // cases of 128^2 618 and 753, 16 of them 120 and 97, 56 of 64^2 64 and 90; Gauss-Seidel, 64
+    // cases of 128^2 405 and 302, of 64^2 77 and 104.)
+    bool band_default(int ig, int G, int blk, int smem) const
     {
         if (x->opt.precision == MGFVM_PREC_MIXED) return x->ncases >= BAND_MIN_CASES;
-        return G <= 2 && x->ncases >= 2 * BAND_MIN_CASES;
+        const int nc = x->ncases, mu = x->sched.nswpm, pu = x->sched.nswpp;
+        const bool jac = x->sched.isolve == MGFVM_JACOBI;
+        auto slots = x->band_slots.find({G, blk, smem});
+        if (slots == x->band_slots.end())
+            slots = x->band_slots.insert({{G, blk, smem}, std::max(1, band_clusters(x->sched.isolve, G, blk, smem))}).first;
+        const int waves = (nc + slots->second - 1) / slots->second;
+        int mx, my;
+        whole_level(ig, mx, my);
+        const double kcells = 1e-3 * (mx - 2) * (my - 2) * nc;
+        const double size = 0.5 + 0.5 * blk / SMOOTH_BLOCK;
+        double band, tiles;
+        if (jac) {
+            const int u = mu + pu;
+            band = waves * size * (56.5 + 1.12 * u) - 8.0;
+            tiles = kcells * (0.235 + 0.0105 * u);
+        } else {
+            QPlan p;
+            double blocks, pairs;
+            band = 1.06 * (waves * size * (58.5 + 1.0 * (2 * mu + 2 * pu)) - 6.0);
+            tiles = 6.0 + 0.13 * kcells;
+            if (mu > 0) {
+                smooth_times(ig, 3, 2 * mu, true, p, blocks, pairs);
+                tiles += std::min(blocks, pairs);
+            }
+            smooth_times(ig, 1, 2 * pu, true, p, blocks, pairs);
+            tiles += std::min(blocks, pairs);
+        }
+        return band < tiles;
     }
     // every case that has level ig has it at mx x my
     bool one_size(int ig, int mx, int my) const
@@ -380,6 +413,13 @@ struct Builder {
         if (x->sched.isolve != MGFVM_GAUSS_SEIDEL || x->tune.smooth_threads[ig] || x->tune.smooth_units[ig] ||
             x->tune.smooth_tma[ig] == 2)
             return false;
+        double t_best, t_old;
+        smooth_times(ig, neq, units, tmp_ok, best, t_best, t_old);
+        return t_best < t_old;
+    }
+    // its time with the best plan, and that of k_smooth's tiles
+    void smooth_times(int ig, int neq, int units, bool tmp_ok, QPlan &best, double &t_best, double &t_old) const
+    {
         int wi = 0, wj = 0;
         for (const mgfvm_config &c : x->cfg)
             if (ig < c.ngrid) {
@@ -403,7 +443,7 @@ struct Builder {
         bool even = true;
         for (const mgfvm_config &c : x->cfg) even = even && (ig >= c.ngrid || npx_of(c, ig) % 2 == 0);
         const double later = even ? 3.5 : 4.9;
-        double t_best = 1e300, t_old = 1e300;
+        t_best = t_old = 1e300;
         int dummy;
         for (int c = 1; c <= units; ++c) {
             if ((c & 1) && !tmp_ok && c < units) continue;      // an odd count needs a copy back
@@ -423,7 +463,6 @@ struct Builder {
         }
         const PairShape p = pair_shape(ig, units, SMOOTH_BLOCK / 2, tmp_ok);
         if (small_blocks(ig, neq, p.tile)) t_old = std::min(t_old, 0.3 + p.chunks * (1.3 + 0.3 * p.hmax));
-        return t_best < t_old;
     }
     // Mixed precision's plan (k_smooth_q32), any number of launches; false where the tuning asks
     // for k_smooth_f32's.  Its times, 4 us a round of CTAs (two an SM) and 0.2 a unit, choose

@@ -1982,6 +1982,29 @@ int smooth_pairs_side(int units, int threads)
     return s - 2 * units;
 }
 
+int band_clusters(int isolve, int G, int block, int smem)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)G;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)G, 1, 1);
+    c.blockDim = dim3((unsigned)block, 1, 1);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.attrs = at;
+    c.numAttrs = 1;
+    int n = 0;
+    const cudaError_t e = isolve == MGFVM_JACOBI ? cudaOccupancyMaxActiveClusters(&n, k_band_visit<MGFVM_JACOBI>, &c)
+                                                 : cudaOccupancyMaxActiveClusters(&n, k_band_visit<MGFVM_GAUSS_SEIDEL>, &c);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 cudaError_t configure_kernels()
 {
     cudaError_t e = configure_smooth_q();

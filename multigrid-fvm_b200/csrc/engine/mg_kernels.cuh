@@ -86,10 +86,12 @@ constexpr int VISIT_SMEM_MAX = 7 * 2 * SMOOTH_BLOCK * (int)sizeof(double);
 constexpr int BAND_MAX_CTAS = 8;
 constexpr int BAND_SMEM_MAX = 80 * 1024;
 // By default a mixed-precision context runs band visits in batches of at least this many
-// cases (of one size at the level), an FP64 one in larger ones (band_default): a unit costs
-// about a microsecond there (its cluster barrier), which only pays when the tile launches it
-// replaces have enough work to be slow too
+// cases (of one size at the level), an FP64 one where they are expected to be the faster
+// (band_default): a unit costs about a microsecond there (its cluster barrier), which only
+// pays when the tile launches it replaces have enough work to be slow too
 constexpr int BAND_MIN_CASES = 32;
+// clusters of G CTAs of k_band_visit the current device holds at a time (0: unknown)
+int band_clusters(int isolve, int G, int block, int smem);
 // interior rows of each band when G CTAs share a level of npy padded rows (even; the
 // last band may be shorter)
 __host__ __device__ __forceinline__ int band_rows(int npy, int G)
