@@ -350,11 +350,6 @@ __device__ __forceinline__ typename IO::T cell_mass_coefp_io(const IO &io, const
     }
     return ad;
 }
-__device__ __forceinline__ double cell_mass_coefp(const LevelDev &L, const CaseDev &C, int i, int j,
-                                                  bool from_tmp = false)
-{
-    return cell_mass_coefp_io(Prim{L}, C, i, j, from_tmp);
-}
 
 // update :1127-1152 (the obstacle pressure copy :1153-1177 is a separate gather);
 // `parts` bits 1, 2, 4 select the u, v, p updates (each reads only its own operands)
@@ -369,7 +364,6 @@ __device__ __forceinline__ void cell_update_io(const IO &io, const CaseDev &C, i
         io.st(S_V, q, io.ld(S_V, q) + io.g(S_AREAY, q) * (ppq - io.ld(S_PP, q + io.L.npx)) / io.ld(S_APV, q));
     if (parts & 4) io.st(S_P, q, io.ld(S_P, q) + C.relxp * (ppq - ppref));
 }
-__device__ __forceinline__ void cell_update(const LevelDev &L, const CaseDev &C, int q) { cell_update_io(Prim{L}, C, q); }
 
 // --------------------------------------------------------------- smoothers
 __device__ __forceinline__ int eq_field(int e) { return e == EQ_U ? S_U : e == EQ_V ? S_V : e == EQ_PP ? S_PP : S_SC; }
@@ -511,11 +505,6 @@ __device__ __forceinline__ void cell_gs_io(const IO &io, int e, int phi, int q)
                    io.ld(co_slot(e, CK_AN), q), io.ld(co_slot(e, CK_AP), q), io.ld(co_slot(e, CK_SU), q),
                    io.ld(phi, q - 1), io.ld(phi, q + 1), io.ld(phi, q - nx), io.ld(phi, q + nx)));
 }
-__device__ __forceinline__ void cell_jacobi(const LevelDev &L, int e, int cur, int nxt, int q)
-{
-    cell_jacobi_io(Prim{L}, e, cur, nxt, q);
-}
-__device__ __forceinline__ void cell_gs(const LevelDev &L, int e, int phi, int q) { cell_gs_io(Prim{L}, e, phi, q); }
 
 // ------------------------------------------------------------ restriction
 // restv :1354-1389 at coarse interior cell (ic, jc); `parts` bits 1, 2, 4, 8 select
@@ -542,10 +531,6 @@ __device__ __forceinline__ void cell_restv_io(const IO &F, const IO &K, int ic, 
     if (parts & 2) K.st(S_RV, qc, v);
     if (parts & 4) K.st(S_RP, qc, p);
     if (parts & 8) K.st(S_RSC, qc, sc);
-}
-__device__ __forceinline__ void cell_restv(const LevelDev &F, const LevelDev &K, int ic, int jc)
-{
-    cell_restv_io(Prim{F}, Prim{K}, ic, jc);
 }
 
 // residual of the u equation at face (i, j) (restru :1494-1512 fine, :1528-1541 coarse)
@@ -614,10 +599,6 @@ __device__ __forceinline__ void cell_fine_residuals_io(const IO &F, const CaseDe
     if (which == 1 && j <= ny - 3) F.st(S_TMP1, q, resid_v(F, C, ff, i, j, true));
     if (which == 2) F.st(S_TMP2, q, resid_sc(F, ff, i, j, true));
 }
-__device__ __forceinline__ void cell_fine_residuals(const LevelDev &F, const CaseDev &C, int i, int j, int which)
-{
-    cell_fine_residuals_io(Prim{F}, C, i, j, which);
-}
 
 // FAS defects at coarse cell (ic, jc): restru :1546-1563 (which 0), restrv :1722-1738
 // (1), restrsc :1634-1647 (2), from the fine residuals above and the coarse
@@ -649,11 +630,6 @@ __device__ __forceinline__ void cell_restrict_io(const IO &F, const IO &K, const
         T rc = resid_sc(K, fk, ic, jc, false);
         K.st(S_RESSC, qc, (F.ld(r, q) + F.ld(r, q - nxf) + F.ld(r, q - 1) + F.ld(r, q - 1 - nxf)) - rc);
     }
-}
-__device__ __forceinline__ void cell_restrict(const LevelDev &F, const LevelDev &K, const CaseDev &C, int ic, int jc,
-                                              int which)
-{
-    cell_restrict_io(Prim{F}, Prim{K}, C, ic, jc, which);
 }
 
 // ---------------------------------------------------------- prolongation
@@ -839,7 +815,6 @@ __device__ __forceinline__ void row_periodic_x_io(const IO &io, int j)
     io.st(S_U, q, io.ld(S_U, q1)); io.st(S_U, q1 + 1, io.ld(S_U, q + 1));
     io.st(S_V, q, io.ld(S_V, q1)); io.st(S_V, q1 + 1, io.ld(S_V, q + 1));
 }
-__device__ __forceinline__ void row_periodic_x(const LevelDev &L, int j) { row_periodic_x_io(Prim{L}, j); }
 
 // pbound y-periodic :1197-1208; sequential: later iterations read cells earlier
 // iterations wrote (the reference's flat offset i + npy - 3), so one thread runs it.
@@ -853,6 +828,5 @@ __device__ __forceinline__ void line_periodic_y_io(const IO &io)
         io.st(S_V, q, io.ld(S_V, q1)); io.st(S_V, q1 + nx, io.ld(S_V, q + nx));
     }
 }
-__device__ __forceinline__ void line_periodic_y(const LevelDev &L) { line_periodic_y_io(Prim{L}); }
 
 }  // namespace mg
