@@ -149,7 +149,12 @@ typedef struct mgfvm_tuning {
     int smooth_units[MGFVM_MAX_LEVELS];    /* smoother units (GS half-sweeps or Jacobi
                                               sweeps) per tile launch, >= 1             */
     int smooth_threads[MGFVM_MAX_LEVELS];  /* smoother CTA: 1024 (one per SM), 512 (two)
-                                              or 256 threads (four)                     */
+                                              or 256 threads (four).  Either of these two
+                                              not 0 also chooses the smoother that gives a
+                                              thread a pair of cells; with both 0 the
+                                              schedule chooses between that one and the
+                                              one by blocks of 2 x 4 cells, with its
+                                              launches and tiles, by expected time       */
     int asm_slices[MGFVM_MAX_LEVELS];      /* assembly threads per cell, 1 or 3, that share
                                               nothing; 0: by tiles through shared memory */
     int restrict_slices[MGFVM_MAX_LEVELS]; /* the same for the restriction              */

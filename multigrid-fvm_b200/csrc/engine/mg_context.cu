@@ -4,7 +4,7 @@
 // the launch schedule of one V-cycle (Version-6-26-04.c:195-249) once, captures it
 // in a CUDA graph and replays that graph; the stop rule is evaluated on the device
 // at the end of every cycle, so the host only polls per-case flags every
-// `sync_every` cycles and a converged case costs nothing but early-exiting blocks.
+// `sync_every` cycles and a converged case costs little but early-exiting blocks.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -672,7 +672,8 @@ struct Builder {
     }
     // Whether the launch about to be added follows a smoother launch (or the copy back
     // of its buffers), with programmatic dependent launch on: masserror+coefp and update
-    // then read the operands that smoothers do not write before waiting for it.
+    // then read the operands that smoothers do not write before waiting for it (the rule
+    // for such reads: pdl_enter, mg_grid.cuh).
     bool after_smoother(int mode) const
     {
         if (!x->sched.pdl || mode == M_OP || out->empty()) return false;

@@ -40,11 +40,16 @@ static __device__ __forceinline__ int nth_eq(int mask, int k)
 // ---------------------------------------------- programmatic dependent launch
 // The V-cycle's kernels are launched with programmatic stream serialization (when the
 // schedule's `pdl` switch is on), so a kernel's CTAs may be scheduled while its
-// predecessor is still running.  Every kernel therefore starts by waiting until the
-// grids it depends on have completed and their memory is visible (a no-op for a
-// kernel launched without the attribute), and then lets its own dependent launch
-// begin: at most one kernel waits ahead of the running one, and nothing a kernel
-// reads or writes is touched before its predecessors are done.
+// predecessor is still running.  Two rules keep that in order:
+//   * every thread waits (pdl_enter: until the launch before has completed and its writes
+//     are visible; a no-op without the attribute) before the kernel's own dependent launch
+//     is let begin, so all launches but the one directly before have completed by then;
+//   * before that wait a kernel writes nothing, and reads only what the launch directly
+//     before it does not write: its level's description and masks, case state that only
+//     other launches set (stopped_before), and in the EARLY instantiations operands, where
+//     the schedule says which launch comes before (after_smoother and the launches of one
+//     smoothing, mg_context.cu).  A launch put in between, or a kernel that lets its
+//     dependents begin before its own wait, breaks this silently.
 static __device__ __forceinline__ void pdl_enter()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
