@@ -109,17 +109,25 @@ def load_peaks():
         return {}
 
 
-# DRAM bytes (read + write) per k_smooth launch of the p' smoothing on level 0, from ncu
-# captures (profiles/k_smooth_obstacle256.md): the 2-case workload of
-# `python bench.py --profile-cycles 1`, and the 64-case batch of the `batched` entry.
-ROOFLINE_TRAFFIC = {"c1": 7475712, "c1x64": 266211072}
+# DRAM bytes (read + write) per launch of the p' smoothing on level 0, from ncu captures
+# (profiles/smoothers_obstacle256.md) by workload and kernel.
+ROOFLINE_TRAFFIC = {}
 
 
-def smoother_roofline(solver, cases, traffic=None, reps=20):
-    """Roofline entry of k_smooth: the p' smoothing of level 0 (nswpp red-black sweeps,
-    split into launches of up to 10 half-sweeps each), timed with CUDA events on the
-    context stream.  Algorithmic bytes: 64 B per cell-sweep (6 coefficients + phi read
-    + phi write, FP64) x nswpp x interior cells, per launch."""
+def op_smoother(solver, level=0):
+    """The kernel mgfvm_time_op's smoothing of `level` runs: the V-cycle's own, except that
+    an op's launches of k_smooth_q have a CTA a tile however many tiles there are (the
+    V-cycle's go through a table of them where there are more than SMs, k_smooth_qs)."""
+    kernels = {k for k, lv, _ in solver.profile_cycle() if lv == level and k.startswith("smooth")}
+    return "k_" + (kernels.pop() if len(kernels) == 1 else "smooth")
+
+
+def smoother_roofline(solver, cases, workload=None, reps=20):
+    """Roofline entry of the level-0 smoother: the p' smoothing (nswpp red-black sweeps,
+    split into launches as the schedule says), timed with CUDA events on the context
+    stream.  Algorithmic bytes: 64 B per cell-sweep (6 coefficients + phi read + phi
+    write, FP64) x nswpp x interior cells, per launch."""
+    kernel = op_smoother(solver)
     solver.time_op("smooth_pp", 0, 2)
     kms, klaunch = solver.time_op("smooth_pp", 0, reps)
     per_launch_ms = kms / klaunch
@@ -129,8 +137,8 @@ def smoother_roofline(solver, cases, traffic=None, reps=20):
     peak = peaks.get("hbm_gbs", 6650.0)
     achieved = algo_bytes / (per_launch_ms / 1e3) / 1e9
     return {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "traffic": traffic,
-            "kernel": "Gauss-Seidel tile smoother (k_smooth_q; k_smooth under a tuned schedule), p' equation, level 0",
+            "frac": round(achieved / peak, 4), "traffic": ROOFLINE_TRAFFIC.get((workload, kernel)),
+            "kernel": f"{kernel} (tile smoother), p' equation, level 0",
             "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
             "per_launch_us": round(per_launch_ms * 1e3, 3), "launches_per_op": klaunch // reps,
             "algorithmic_bytes_per_launch": int(algo_bytes)}
@@ -162,7 +170,7 @@ def batched_rate(nb, device, tune, cycles_per_solve, ncyc=40):
                                              "frac": round(gbs / peak, 4),
                                              "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}}
             if n > 1:   # level-0 fields of the batch exceed L2: the smoother against HBM
-                out[label]["smoother_roofline"] = smoother_roofline(s, cases, ROOFLINE_TRAFFIC.get(f"c1x{n}"))
+                out[label]["smoother_roofline"] = smoother_roofline(s, cases, f"c1x{n}")
     out["speedup_per_case"] = round(out["batch"]["case_cycles_per_s"] / out["one_case"]["case_cycles_per_s"], 2)
     out["note"] = (f"{ncyc} graph-replayed V-cycles timed with CUDA events after 3 warm-up cycles; "
                    f"solves/s = case-cycles/s / {max(cycles_per_solve)} cycles per solve")
@@ -451,8 +459,9 @@ def cpu_sample(cases, cycles_to_converge, ncyc, procs):
 def run_reference_arm(a, rank, world):
     if rank != 0:
         return
-    # the reference reads the workload's own InputData/pattern.txt directories; nothing
-    # of this package's native code is loaded
+    # the reference reads the workload's own InputData/pattern.txt directories.  Where its
+    # build is not at hand the C restatement of it runs instead (`kind`: port), with this
+    # package's parser reading those files
     if a.workload in WORKLOAD_DIRS:
         cases, nvcycle, desc = WORKLOAD_DIRS[a.workload], [2000, 2000], WORKLOAD_DESC[a.workload]
     else:
@@ -674,7 +683,7 @@ def main():
     cell_sweeps_per_s = sweeps * a.steps * world / (ms / 1e3)
 
     # ---- dominant kernel: the shared-memory tile smoother on level 0, p' equation (live)
-    roofline = smoother_roofline(solver, cases, ROOFLINE_TRAFFIC.get(a.workload))
+    roofline = smoother_roofline(solver, cases, a.workload)
 
     # ---- end to end through the public API with host buffers
     e2e = None
