@@ -111,23 +111,24 @@ def load_peaks():
 
 # DRAM bytes (read + write) per launch of the p' smoothing on level 0, from ncu captures
 # (profiles/smoothers_obstacle256.md) by workload and kernel.
-ROOFLINE_TRAFFIC = {}
+ROOFLINE_TRAFFIC = {("c1", "k_smooth"): 7428352, ("c1", "k_smooth_q"): 7487488,
+                    ("c1x64", "k_smooth"): 266097152, ("c1x64", "k_smooth_q"): 266439168}
 
 
 def op_smoother(solver, level=0):
     """The kernel mgfvm_time_op's smoothing of `level` runs: the V-cycle's own, except that
     an op's launches of k_smooth_q have a CTA a tile however many tiles there are (the
-    V-cycle's go through a table of them where there are more than SMs, k_smooth_qs)."""
+    V-cycle's go through a table of them where there are more than SMs, k_smooth_qs).
+    Runs a V-cycle: for before the timed solves, which start from a reset."""
     kernels = {k for k, lv, _ in solver.profile_cycle() if lv == level and k.startswith("smooth")}
     return "k_" + (kernels.pop() if len(kernels) == 1 else "smooth")
 
 
-def smoother_roofline(solver, cases, workload=None, reps=20):
+def smoother_roofline(solver, cases, kernel, workload=None, reps=20):
     """Roofline entry of the level-0 smoother: the p' smoothing (nswpp red-black sweeps,
     split into launches as the schedule says), timed with CUDA events on the context
     stream.  Algorithmic bytes: 64 B per cell-sweep (6 coefficients + phi read + phi
     write, FP64) x nswpp x interior cells, per launch."""
-    kernel = op_smoother(solver)
     solver.time_op("smooth_pp", 0, 2)
     kms, klaunch = solver.time_op("smooth_pp", 0, reps)
     per_launch_ms = kms / klaunch
@@ -156,6 +157,7 @@ def batched_rate(nb, device, tune, cycles_per_solve, ncyc=40):
         with Solver(cases, device=device, sync_every=64) as s:
             if tune:
                 s.autotune(3)
+            kernel = op_smoother(s)
             s.cycle(3)
             s.cycle(ncyc)
             ms = s.last_elapsed_ms / ncyc
@@ -170,7 +172,7 @@ def batched_rate(nb, device, tune, cycles_per_solve, ncyc=40):
                                              "frac": round(gbs / peak, 4),
                                              "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"}}
             if n > 1:   # level-0 fields of the batch exceed L2: the smoother against HBM
-                out[label]["smoother_roofline"] = smoother_roofline(s, cases, f"c1x{n}")
+                out[label]["smoother_roofline"] = smoother_roofline(s, cases, kernel, f"c1x{n}")
     out["speedup_per_case"] = round(out["batch"]["case_cycles_per_s"] / out["one_case"]["case_cycles_per_s"], 2)
     out["note"] = (f"{ncyc} graph-replayed V-cycles timed with CUDA events after 3 warm-up cycles; "
                    f"solves/s = case-cycles/s / {max(cycles_per_solve)} cycles per solve")
@@ -612,6 +614,7 @@ def main():
             log(f"  {k:22s} x{c:3d} {v * 1e3:9.1f} us  {100 * v / tot:5.1f}%  avg {v / c * 1e3:7.2f} us")
         solver.close()
         return
+    kernel = op_smoother(solver)
     stream = torch.cuda.ExternalStream(solver.stream, device=torch.device("cuda", local))
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
 
@@ -683,7 +686,7 @@ def main():
     cell_sweeps_per_s = sweeps * a.steps * world / (ms / 1e3)
 
     # ---- dominant kernel: the shared-memory tile smoother on level 0, p' equation (live)
-    roofline = smoother_roofline(solver, cases, a.workload)
+    roofline = smoother_roofline(solver, cases, kernel, a.workload)
 
     # ---- end to end through the public API with host buffers
     e2e = None
