@@ -2037,7 +2037,8 @@ int mgfvm_autotune(mgfvm_ctx *x, int cycles, mgfvm_tuning *chosen, double *ms_be
     int rc = MGFVM_OK;
     double t0 = 0.0, best = 0.0;
     auto trial = [&](double *ms) -> int {
-        x->hs = saved;                  // histories and flags as before every trial
+        x->hs = saved;                  // histories as before every trial, and every case running
+        for (CaseState &S : x->hs) S.done = S.gone = 0;
         RC(push(x));
         return time_schedule(x, cycles, ms);
     };
