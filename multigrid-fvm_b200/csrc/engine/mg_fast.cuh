@@ -42,7 +42,9 @@ __device__ __forceinline__ FastLevel fast_level(const LevelDev &L)
 
 // Begins the loads of a kernel's description here, ahead of a branch on the case's stop
 // flag, which the compiler would otherwise have them wait for: a V-cycle of 64 256^2 cases
-// 2.295 ms against 2.344 (and 2.323 with no such branch).
+// 2.264 ms against 2.311 with the assembly without it, 2.285 with the update.  (In the
+// residual, the prolongation and the pair smoother it costs registers or time and is left
+// out: 2.264 to 2.254 for the residual, 2.269 to 2.262 for the prolongation.)
 __device__ __forceinline__ void begin_loads(const CaseDev &C, const FastLevel &L)
 {
     asm volatile("" ::"r"(L.npx), "r"(L.npy), "r"(L.sb), "l"(L.b), "r"(C.ngrid), "r"(C.tail));

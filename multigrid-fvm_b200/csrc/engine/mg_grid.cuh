@@ -61,7 +61,7 @@ static __device__ __forceinline__ void pdl_enter()
 // the first launch of level 0 (that takes `gone`, or reads `done` after its wait) or by an
 // op.  The blocks of a stopped case end there, before they load anything: a cycle of 64
 // stopped 256^2 cases takes 0.28 ms against 1.52 where the flag was read along with the
-// data, of two 60 us against 115 (a running one 2.29 ms and 228 us).
+// data, of two 52 us against 115 (a running one 2.25 ms and 227 us).
 static __device__ __forceinline__ bool stopped_before(const CaseState &S, int mode)
 {
     return (S.done != 0) & (mode > M_OP_C);

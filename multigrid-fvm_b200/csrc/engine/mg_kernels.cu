@@ -273,7 +273,6 @@ __global__ void __launch_bounds__(BLOCK, EARLY ? 5 : 4) k_mass_coefp(const CaseD
     const Fast io{L};
     const int n = (L.npx - 2) * (L.npy - 2), nb = (n + blockDim.x - 1) / blockDim.x;
     const bool stopped = stopped_before(ST, mode);
-    begin_loads(C, L);
     if (stopped) {
         pdl_enter();
         return;

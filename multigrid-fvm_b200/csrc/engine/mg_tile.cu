@@ -378,11 +378,9 @@ __global__ void __launch_bounds__(NT, 4) k_tile_prol(const CaseDev *__restrict__
     const CaseDev &C = cs[blockIdx.y];
     const FastLevel L = fast_level(C.lv[ig]), LK = fast_level(C.lv[ig + 1]);
     const Fast F{L}, K{LK};
-    begin_loads(C, LK);
     const int nx = L.npx, ny = L.npy, nxc = LK.npx, nyc = LK.npy, t = threadIdx.x, txn = max(1, (nx - 2 + TX - 1) / TX);
     const int i0 = 1 + (blockIdx.x % txn) * TX, j0 = 1 + (blockIdx.x / txn) * TY;
     const bool stopped = stopped_before(st[blockIdx.y], mode);
-    begin_loads(C, L);
     if (stopped) {
         pdl_enter();
         return;
