@@ -143,7 +143,8 @@ typedef struct mgfvm_options {
 } mgfvm_options;
 
 /* Per-level schedule choices (index = level; 0 = the engine's default).  Every choice
- * gives the same bits; only the launch shapes change. */
+ * gives the same bits in FP64; only the launch shapes change.  (In mixed precision a level
+ * of band visits is smoothed in FP64, one of tiles in FP32.) */
 #define MGFVM_MAX_LEVELS 16
 typedef struct mgfvm_tuning {
     int smooth_units[MGFVM_MAX_LEVELS];    /* smoother units (GS half-sweeps or Jacobi
