@@ -350,7 +350,7 @@ struct Builder {
         if (jac) {
             const int u = mu + pu;
             band = waves * size * (56.5 + 1.12 * u) - 8.0;
-            tiles = kcells * (0.235 + 0.0105 * u);
+            tiles = 4.0 + kcells * (0.235 + 0.0105 * u);
         } else {
             QPlan p;
             double blocks, pairs;
